@@ -57,6 +57,16 @@ struct MixedSys;
 struct SweepSys;
 struct Scene;
 
+// The shape of a scene's chip-resident PCG solve (od_resident.cu); warps 0:
+// the system is too large for it.
+struct ResidentPlan {
+  int grid = 0, warps = 0, bytes = 0;   // CTAs; worker warps and dynamic shared memory of each
+  bool smem = false;                    // the matrix in shared memory, else in ell
+  std::vector<int> off;                 // not smem: first matrix step of every CTA in ell
+  unsigned char* ell = nullptr;
+  int* ell_off = nullptr;               // off on the device
+};
+
 struct Pcg {
   int n_pad = 0;
   int precision = OD_PRECISION_FP64;
@@ -128,6 +138,7 @@ struct Pcg {
   int recur = -1;               // one-launch PCG form: 1 recurrence (q = A z + beta q; two grid syncs),
                                 // 0 the reference's (q = A p; three), -1 chosen by the tolerance
   int disable_persistent = 0;
+  ResidentPlan res;
   // mixed precision: the scene's sliced FP32 operator and its one-scene
   // solve (both built on first use)
   SliceSys* slice = nullptr;
@@ -594,6 +605,10 @@ od_status mixed_ic0_solve(Scene* s, const double* d_b, double* d_x, const od_sol
                           od_solve_stats* st);
 
 // PCG on A64; b and x are device vectors of length n_pad
+od_status resident_plan(Scene* s);
+void resident_free(ResidentPlan* R);
+od_status resident_solve(Scene* s, const double* d_b, double* d_x, int pkind, double tol, int max_iter, bool x_zero,
+                         unsigned long long* prof);
 od_status pcg_solve(Scene* s, const double* d_b, double* d_x, const od_solver_params* prm, od_solve_stats* st);
 
 // ---- mixed-precision systems (od_sparse.cu)

@@ -2664,6 +2664,7 @@ od_status pcg_alloc(Scene* s) {
   OD_CUDA(cudaFree(P.partial));
   OD_CUDA(cudaMalloc(&P.partial, sizeof(double) * 4 * (size_t)P.grid));
   s->device_bytes += (long long)sizeof(double) * (6 * nv + 9 * (size_t)s->bsr.nb + 4 * (size_t)P.grid);
+  OD_TRY(resident_plan(s));
   return OD_OK;
 }
 
@@ -2682,6 +2683,7 @@ void pcg_free(Scene* s) {
   mixed_ic0_free(P.mic);
   slice_free(P.slice);
   sweep_free(P.sweep);
+  resident_free(&P.res);
   if (P.sc_host) cudaFreeHost(P.sc_host);
   if (P.timeout_host) cudaFreeHost(P.timeout_host);
   cudaFree(P.prof);
@@ -3390,6 +3392,11 @@ od_status pcg_solve(Scene* s, const double* d_b, double* d_x, const od_solver_pa
     unsigned long long* profp = phases ? P.prof : nullptr;
     args[17] = (void*)&profp;
     if (prof) OD_CUDA(cudaEventRecord(s->ctx->ev_pool[0], strm));
+    if (recur == 2 && P.res.warps > 0) {
+      OD_TRY(resident_solve(s, d_b, d_x, pk, prm->tol, prm->max_iter, x_zero, profp));
+      if (prof) OD_CUDA(cudaEventRecord(s->ctx->ev_pool[1], strm));
+      return pcg_finish(s, d_b, d_x, shift, st, true, prof, phases);
+    }
     OD_KL(s);
     OD_CUDA(cudaLaunchCooperativeKernel(fn, dim3(G2), dim3(kPThreads), args, dyn, strm));
     if (prof) OD_CUDA(cudaEventRecord(s->ctx->ev_pool[1], strm));
