@@ -62,7 +62,10 @@ struct Scene;
 struct ResidentPlan {
   int grid = 0, warps = 0, bytes = 0;   // CTAs; worker warps and dynamic shared memory of each
   bool smem = false;                    // the matrix in shared memory, else in ell
+  bool cluster = false;                 // the CTAs are one cluster, else a cooperative grid
   std::vector<int> off;                 // not smem: first matrix step of every CTA in ell
+  void* ctr = nullptr;                  // barrier and sum counters
+  void* mx = nullptr;                   // digits of the gathered vector, two buffers
   unsigned char* ell = nullptr;
   int* ell_off = nullptr;               // off on the device
 };

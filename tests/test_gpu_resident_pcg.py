@@ -1,9 +1,11 @@
-"""The chip-resident FP64 PCG (od_resident.cu) at the edges of its shapes: less than one group of block rows, several
-groups on one CTA, the first system that takes the grid, more than one group per CTA, and the matrix in L2.
+"""The chip-resident FP64 PCG (od_resident.cu) at the edges of its shapes: less than one group of block rows, the most
+one CTA takes, clusters of 2, 4 and 16 CTAs (with CTAs that hold fewer groups than others), the grid, and the matrix in L2.
 
 Bounds: the stop test is on the recursive residual, which a pipelined recurrence keeps within a few hundred roundings of
 the true one over these some hundred iterations, so ||b - A x|| <= (1e-9 + 1e-12) ||b|| with A x by the oracle; iteration
 counts as the other PCG paths' tests hold them (the larger of 2 and 3%)."""
+import functools
+
 import numpy as np
 import pytest
 
@@ -13,10 +15,11 @@ from tests.gpu_util import ctx
 
 pytestmark = pytest.mark.gpu
 
-# free block rows: 4; 36; 120 (the most one CTA takes); 125 (the first on the grid); 1620 (two groups on some CTAs)
-MESHES = [(1, 1, 1), (4, 2, 2), (10, 3, 2), (5, 4, 4), (20, 8, 8)]
+# free block rows: 4; 36 and 40 (one CTA); 48 (two); 120 and 125 (four); 1620 (sixteen); 2400 (the grid)
+MESHES = [(1, 1, 1), (4, 2, 2), (10, 1, 1), (4, 3, 2), (10, 3, 2), (5, 4, 4), (20, 8, 8), (24, 9, 9)]
 
 
+@functools.lru_cache(maxsize=None)
 def system(dims):
     g = meshgen.tet_grid(*dims, h=0.05, jitter=0.15, seed=4)
     cd = meshgen.constrained_dofs_for_nodes(g.face_nodes(0, 0))
@@ -49,7 +52,7 @@ def test_resident_pcg_at_its_edges(dims, precond, smem, monkeypatch):
     assert abs(st.iterations - its) <= max(2, 0.03 * its)
 
 
-@pytest.mark.parametrize("dims", [(4, 2, 2), (20, 8, 8)])
+@pytest.mark.parametrize("dims", [(4, 2, 2), (20, 8, 8), (24, 9, 9)])
 def test_resident_pcg_exits(dims):
     g, cd, _o, A, b = system(dims)
     s = scene(g, cd)
