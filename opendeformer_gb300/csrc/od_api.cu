@@ -311,7 +311,7 @@ static od_status scene_build(Scene* s, int n_nodes, const double* X, int n_tets,
   OD_TRY(dupload(s, &s->node_dof, s->hnode_dof.data(), s->hnode_dof.size()));
   OD_TRY(dupload(s, &s->facets_dev, s->hfacets.data(), s->hfacets.size()));
   OD_TRY(dalloc(s, &s->node_vol4, (size_t)n_nodes));
-  s->n_pre = s->mat.kind == OD_MATERIAL_COROTATIONAL ? 100 : (s->mat.kind == OD_MATERIAL_COROTATIONAL_PLASTIC ? 112 : 22);
+  s->n_pre = element_precomputes();
   OD_TRY(dalloc(s, &s->pre, (size_t)s->n_pre * ne));
   if (s->mat.kind == OD_MATERIAL_COROTATIONAL_PLASTIC) {  // zero plastic strain (corotationalPlastic.cpp:46-47)
     OD_TRY(dalloc(s, &s->plastic, 9 * (size_t)ne));
@@ -480,10 +480,7 @@ od_status od_scene_evaluate(od_scene* scene, double* values, double* f_int) {
   OD_CHECK_ARG(scene, "od_scene_evaluate: scene is NULL");
   Scene* s = &scene->s;
   OD_CUDA(cudaSetDevice(s->ctx->device));
-  // OD_GB300_ELEMENT_DF=1: the mixed-precision path's double-float stiffness
-  // contraction (to compare it with the FP64 one)
-  const char* dfe = std::getenv("OD_GB300_ELEMENT_DF");
-  OD_TRY(launch_eval(s, true, dfe && dfe[0] == '1'));
+  OD_TRY(launch_eval(s, true));
   if (values) OD_CUDA(cudaMemcpyAsync(values, s->K, sizeof(double) * s->nvals, cudaMemcpyDeviceToHost, s->ctx->stream));
   if (f_int) OD_CUDA(cudaMemcpyAsync(f_int, s->fint, sizeof(double) * s->dofs, cudaMemcpyDeviceToHost, s->ctx->stream));
   OD_TRY(sync_stream(s));
@@ -710,7 +707,7 @@ static od_status be_step(Scene* s, od_step_stats* acc) {
   const int n = s->dofs, T = 256;
   cudaStream_t st = s->ctx->stream;
   const double h = p.dt;
-  OD_TRY(launch_eval(s, true, p.solver.precision == OD_PRECISION_MIXED));
+  OD_TRY(launch_eval(s, true));
   // A0 v with A0 = (h + beta_K) K + alpha_M M + D
   OD_TRY(launch_spmv_lower(s, s->K, h + p.beta_k, s->v, s->M, p.alpha_m, s->v, s->Dm, 1.0, s->v, s->tmp, false));
   OD_KL(s);
@@ -746,7 +743,7 @@ static od_status nm_step(Scene* s, od_step_stats* acc) {
     OD_KL(s);
     nm_stage_kernel<<<nblk(n, T), T, 0, st>>>(n, s->free_pos, bh2, gh, p.alpha_m, s->dp, s->vp, s->a, s->u, s->tmp,
                                               s->tmp2);
-    OD_TRY(launch_eval(s, true, p.solver.precision == OD_PRECISION_MIXED));
+    OD_TRY(launch_eval(s, true));
     // y = M (alpha_M v_k + a_k) + beta_K K v_k (+ D v_k)
     OD_TRY(launch_spmv_lower(s, s->M, 1.0, s->tmp, s->K, p.beta_k, s->tmp2, s->Dm, 1.0, s->tmp2, s->rhs, false));
     OD_KL(s);

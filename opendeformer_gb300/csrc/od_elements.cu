@@ -9,6 +9,7 @@
 // map loads are coalesced.  The staged outputs (the gathered assembly's
 // input) are element-major, grouped by local node block (c_kslot below).
 #include "od_internal.h"
+#include "od_fixed.cuh"
 #include "od_math.cuh"
 
 namespace od {
@@ -42,25 +43,23 @@ __device__ __forceinline__ double tet_vol(V3t<double> a, V3t<double> b, V3t<doub
 }
 
 // ------------------------------------------------------------ precomputes
-// getCorotationalTetElementPrecomputes (tetelement.cpp:501-544) and
-// InvertibleHyperelasticTetElement::getPrecomputes (tetelement.cpp:253-266),
-// written in element (colour) order.
-__global__ void precompute_kernel(int ne, int kind, const int4* __restrict__ tets,
-                                  const double* __restrict__ X, double D0, double D1, double D2,
+// What every material's element kernel reads of the rest shape, per element
+// (structure of arrays, element order): the inverse Dm^-1 of the edge matrix
+// (9) and the volume V.  Row i - 1 of Dm^-1 is the gradient of node i's shape
+// function and node 0's is minus their sum, so the shape derivatives of
+// tetelement.cpp:18-48 (6 V times the gradients) and the corotational rest
+// stiffness K0 (tetelement.cpp:501-544) follow from these ten numbers; storing
+// K0 cost 720 more bytes an element and its rotation 540 multiply-adds.
+constexpr int kPreVol = 9;
+constexpr int kPreCount = 10;
+int element_precomputes() { return kPreCount; }
+
+__global__ void precompute_kernel(int ne, const int4* __restrict__ tets, const double* __restrict__ X,
                                   double* __restrict__ pre) {
   int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= ne) return;
   int4 t = tets[e];
   V3t<double> p0 = ld3(X, t.x), p1 = ld3(X, t.y), p2 = ld3(X, t.z), p3 = ld3(X, t.w);
-  // shape-function gradients scaled by 6V (tetelement.cpp:18-48)
-  V3t<double> da = v_sub(p0, p3), db = v_sub(p1, p3), dc = v_sub(p2, p3), ca = v_sub(p0, p2), cb = v_sub(p1, p2);
-  V3t<double> g[4];
-  if (v_dot(da, v_cross(db, dc)) > 0.0) {
-    g[0] = v_cross(db, dc); g[1] = v_cross(dc, da); g[2] = v_cross(da, db); g[3] = v_cross(cb, ca);
-  } else {
-    g[0] = v_cross(dc, db); g[1] = v_cross(da, dc); g[2] = v_cross(db, da); g[3] = v_cross(ca, cb);
-  }
-  double vol = tet_vol(p0, p1, p2, p3);
   V3t<double> ab = v_sub(p1, p0), ac = v_sub(p2, p0), ad = v_sub(p3, p0);
   double Dm[9] = {ab.x, ac.x, ad.x, ab.y, ac.y, ad.y, ab.z, ac.z, ad.z}, Di[9];
   double inv = 1.0 / det3(Dm);
@@ -73,42 +72,8 @@ __global__ void precompute_kernel(int ne, int kind, const int4* __restrict__ tet
   Di[6] = (Dm[3] * Dm[7] - Dm[4] * Dm[6]) * inv;
   Di[7] = (Dm[1] * Dm[6] - Dm[0] * Dm[7]) * inv;
   Di[8] = (Dm[0] * Dm[4] - Dm[1] * Dm[3]) * inv;
-  if (kind == OD_MATERIAL_COROTATIONAL || kind == OD_MATERIAL_COROTATIONAL_PLASTIC) {
-    const double f = 1.0 / (36.0 * vol);
-    int k = 0;
-    for (int a = 0; a < 4; a++) {
-      const double Ba[3] = {g[a].x, g[a].y, g[a].z};
-      for (int b = a; b < 4; b++) {
-        const double Bb[3] = {g[b].x, g[b].y, g[b].z};
-        pre[(size_t)(k + 0) * ne + e] = (D0 * Ba[0] * Bb[0] + D2 * (Ba[1] * Bb[1] + Ba[2] * Bb[2])) * f;
-        pre[(size_t)(k + 1) * ne + e] = (D1 * Ba[0] * Bb[1] + D2 * Ba[1] * Bb[0]) * f;
-        pre[(size_t)(k + 2) * ne + e] = (D1 * Ba[0] * Bb[2] + D2 * Ba[2] * Bb[0]) * f;
-        pre[(size_t)(k + 3) * ne + e] = (D1 * Ba[1] * Bb[0] + D2 * Ba[0] * Bb[1]) * f;
-        pre[(size_t)(k + 4) * ne + e] = (D0 * Ba[1] * Bb[1] + D2 * (Ba[0] * Bb[0] + Ba[2] * Bb[2])) * f;
-        pre[(size_t)(k + 5) * ne + e] = (D1 * Ba[1] * Bb[2] + D2 * Ba[2] * Bb[1]) * f;
-        pre[(size_t)(k + 6) * ne + e] = (D1 * Ba[2] * Bb[0] + D2 * Ba[0] * Bb[2]) * f;
-        pre[(size_t)(k + 7) * ne + e] = (D1 * Ba[2] * Bb[1] + D2 * Ba[1] * Bb[2]) * f;
-        pre[(size_t)(k + 8) * ne + e] = (D0 * Ba[2] * Bb[2] + D2 * (Ba[0] * Bb[0] + Ba[1] * Bb[1])) * f;
-        k += 9;
-      }
-    }
-    for (int i = 0; i < 9; i++) pre[(size_t)(90 + i) * ne + e] = Di[i];
-    pre[(size_t)99 * ne + e] = vol;
-    if (kind == OD_MATERIAL_COROTATIONAL_PLASTIC)  // shape derivatives for the stress forces
-      for (int a = 0; a < 4; a++) {
-        pre[(size_t)(100 + 3 * a) * ne + e] = g[a].x;
-        pre[(size_t)(101 + 3 * a) * ne + e] = g[a].y;
-        pre[(size_t)(102 + 3 * a) * ne + e] = g[a].z;
-      }
-  } else {
-    for (int a = 0; a < 4; a++) {
-      pre[(size_t)(3 * a) * ne + e] = g[a].x;
-      pre[(size_t)(3 * a + 1) * ne + e] = g[a].y;
-      pre[(size_t)(3 * a + 2) * ne + e] = g[a].z;
-    }
-    for (int i = 0; i < 9; i++) pre[(size_t)(12 + i) * ne + e] = Di[i];
-    pre[(size_t)21 * ne + e] = vol;
-  }
+  for (int i = 0; i < 9; i++) pre[(size_t)i * ne + e] = Di[i];
+  pre[(size_t)kPreVol * ne + e] = tet_vol(p0, p1, p2, p3);
 }
 
 // ------------------------------------------------------------ mass / loads
@@ -116,11 +81,11 @@ __device__ __forceinline__ int local12(int a, int b) { return a * 12 - ((a - 1) 
 
 // consistent mass, rho V / 10 on the diagonal and rho V / 20 off it, same
 // axis only (tetelement.cpp:51-66, mechMaterial.cpp:69-98); one colour
-__global__ void mass_kernel(int e0, int e1, int ne, int vslot, double rho, const double* __restrict__ pre,
+__global__ void mass_kernel(int e0, int e1, int ne, double rho, const double* __restrict__ pre,
                             const int* __restrict__ emap, double* __restrict__ M) {
   int e = e0 + blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= e1) return;
-  double vol = pre[(size_t)vslot * ne + e];
+  double vol = pre[(size_t)kPreVol * ne + e];
   double od = vol * 0.05, dg = vol * 0.1;
   for (int a = 0; a < 4; a++)
     for (int b = a; b < 4; b++) {
@@ -133,12 +98,12 @@ __global__ void mass_kernel(int e0, int e1, int ne, int vslot, double rho, const
 }
 
 // V/4 per incident element, summed per node (body-force weights); one colour
-__global__ void node_vol_kernel(int e0, int e1, int ne, int vslot, const int4* __restrict__ tets,
+__global__ void node_vol_kernel(int e0, int e1, int ne, const int4* __restrict__ tets,
                                 const double* __restrict__ pre, double* __restrict__ nv) {
   int e = e0 + blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= e1) return;
   int4 t = tets[e];
-  double q = pre[(size_t)vslot * ne + e] / 4.0;
+  double q = pre[(size_t)kPreVol * ne + e] / 4.0;
   nv[t.x] += q; nv[t.y] += q; nv[t.z] += q; nv[t.w] += q;
 }
 
@@ -179,275 +144,235 @@ __global__ void loads_kernel(int n, int dofs, const int* __restrict__ free_pos, 
   fext[i] = acc;
 }
 
-// ------------------------------------------------- double-float arithmetic
-// A value as hi + lo of two floats (about 46 significant bits), for the
-// mixed-precision path's element stiffness contraction: on this part the
-// FP64 units run at 1/70 of the FP32 rate and also execute every FP32 <->
-// FP64 conversion, so operands are split and results rebuilt with integer
-// bit operations, and the products and sums run on the FP32 units
-// (error-free TwoProduct by FMA and TwoSum, Dekker / Knuth).
-struct DFv {
-  float hi, lo;
+// ------------------------------------------------------ element stiffness
+// An element's outputs: MODE 1 the packed 12x12 upper triangle in the caller's
+// element order, MODE 2 the colour-ordered staging arrays (node blocks
+// contiguous, c_kslot).
+template <int MODE>
+struct ElemOut {
+  double* k;
+  double* f;
+  __device__ __forceinline__ ElemOut(int e, double* out78, double* out12, const int* perm) {
+    const size_t o = MODE == 1 ? (size_t)perm[e] : (size_t)e;
+    k = out78 + o * 78;
+    f = out12 + o * 12;
+  }
+  // block (a, b), a <= b, row-major; a diagonal block's upper triangle
+  __device__ __forceinline__ void block(int a, int b, const double (&o)[9]) const {
+    if constexpr (MODE == 1) {
+#pragma unroll
+      for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = 0; j < 3; j++)
+          if (a != b || j >= i) k[c_diag12[a * 3 + i] + (b - a) * 3 - i + j] = o[i * 3 + j];
+    } else {
+      // blocks before (a, b): rows 0..a-1 hold 6 + 9 (3 - row) values each
+      const int base = a * 33 - 9 * (a * (a - 1)) / 2 + (b == a ? 0 : 6 + 9 * (b - a - 1));
+      double* p = k + base;
+      if (a == b) {
+        p[0] = o[0];
+        p[1] = o[1];
+        p[2] = o[2];
+        p[3] = o[4];
+        p[4] = o[5];
+        p[5] = o[8];
+      } else if (base & 1) {   // 78 e is even: pairs of values at even places
+        p[0] = o[0];
+#pragma unroll
+        for (int q = 1; q < 9; q += 2) *reinterpret_cast<double2*>(p + q) = make_double2(o[q], o[q + 1]);
+      } else {
+#pragma unroll
+        for (int q = 0; q < 8; q += 2) *reinterpret_cast<double2*>(p + q) = make_double2(o[q], o[q + 1]);
+        p[8] = o[8];
+      }
+    }
+  }
+  __device__ __forceinline__ void forces(const double (&v)[12]) const {
+    double2* p = reinterpret_cast<double2*>(f);
+#pragma unroll
+    for (int q = 0; q < 6; q++) p[q] = make_double2(v[2 * q], v[2 * q + 1]);
+  }
 };
 
-// x = hi + lo + d with |d| <= 2^-47 |x|: hi is x with its significand cut to
-// 24 bits, lo the next 24 bits of the remainder.  Magnitudes below the
-// normal float range give 0; infinities and NaNs pass through hi.
-__device__ __forceinline__ DFv df_split(double x) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-  const unsigned sign = (unsigned)(b >> 32) & 0x80000000u;
-  const int e = (int)((b >> 52) & 0x7FF);
-  const unsigned long long m = b & 0xFFFFFFFFFFFFFull;
-  const int ef = e - 1023 + 127;
-  DFv r{0.f, 0.f};
-  if (ef >= 255) {
-    r.hi = __uint_as_float(sign | (e == 2047 && m ? 0x7FC00000u : 0x7F800000u));
-    return r;
+// The stiffness runs in fixed point (od_fixed.cuh): it is two thirds of an
+// element's arithmetic, a warp-wide FP64 multiply-add holds the SM's FP64 unit
+// for 16 cycles and the three wide integer multiply-adds in its place take 1.5.
+// Every factor of an element has one scale, products keep 60 bits of theirs,
+// and the scales grow by at most 2^7 over a result's own size, so a value
+// carries 2^-53 of the element's largest, where FP64's sums of the same
+// products carry several 2^-53 (assembled matrix of the beam against 64-bit
+// linear algebra, 2-norm: Neo-Hookean 5.9e-16, 5.8e-16 in FP64; corotational
+// 5.0e-16 both).  Exponents outside this window (and NaN and infinities among
+// the factors) take the same sums in FP64.
+// Elements and assembly together, FP64 contraction -> now: Neo-Hookean 98k
+// tets 445 -> 272 us, 655k 2,463 -> 1,375; corotational 416 -> 183 and 2,172 ->
+// 891.  The FP64 unit is about half busy with the decompositions then; what
+// keeps it from more are instruction latency at 16 warps an SM and phases that
+// the warps of one wave pass together.
+constexpr int kElExpMin = 823, kElExpMax = 1223;   // biased: 2^-200 .. 2^200
+constexpr int kElThreads = 128;
+constexpr int kHyperCtas = 4;   // 128 registers a thread: 16 warps on an SM
+
+template <int N>
+__device__ __forceinline__ int max_exp(const double (&v)[N], int e = 0) {
+#pragma unroll
+  for (int i = 0; i < N; i++) e = max(e, fx_biased_exp(v[i]));
+  return e;
+}
+__device__ __forceinline__ bool exp_fits(int e) { return e >= kElExpMin && e <= kElExpMax; }
+
+// Per-thread columns of a CTA's shared memory: rotated gradients as digits
+// (component 3 n + i of node n); the hyperelastic stiffness keeps node 0's row
+// of blocks there too, as sums over the others.
+struct HyperShared {
+  int2 g[12][kElThreads];
+  long long row0[27][kElThreads];
+};
+
+// Gradients of the shape functions in a rotated frame, Q g_n, as digits in
+// this thread's column of sa; returns their scale Ea, with |Q g_n| <
+// 2^(Ea - 1).  q: Q's digits at the scale 1 (orthonormal, row-major); d: those
+// of Di at the scale E, its rows g_1..g_3; node 0's gradient (if asked for) is
+// minus their sum.
+template <bool NODE0>
+__device__ __forceinline__ int fx_gradients(const int2 (&q)[9], const int2 (&d)[9], int E, int2 (*sa)[kElThreads]) {
+  // at the scale E + 1, where node 0's, below 6 2^E, stay under 2^62; then
+  // moved to the scale that leaves the largest one place spare (each place a
+  // factor wastes is lost twice in a stiffness value)
+  long long x[4][3], top = 0;
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    x[0][i] = 0;
+#pragma unroll
+    for (int n = 1; n < 4; n++) {
+      FxAcc c;
+#pragma unroll
+      for (int k = 0; k < 3; k++) c.add(q[i * 3 + k], d[(n - 1) * 3 + k]);
+      x[n][i] = (c.hh + (c.mid >> kFxLow) + 2) >> 2;
+      x[0][i] -= x[n][i];
+    }
+#pragma unroll
+    for (int n = NODE0 ? 0 : 1; n < 4; n++) top |= x[n][i] ^ (x[n][i] >> 63);
   }
-  if (ef <= 0) return r;
-  r.hi = __uint_as_float(sign | ((unsigned)ef << 23) | (unsigned)(m >> 29));
-  const unsigned rem = (unsigned)(m & 0x1FFFFFFFull);   // the remainder, in units of 2^(e-1075)
-  if (rem == 0) return r;
-  const int top = 31 - __clz((int)rem);                  // its leading bit, 0..28
-  const unsigned frac = (top >= 23 ? (rem >> (top - 23)) : (rem << (23 - top))) & 0x7FFFFFu;
-  const int elo = e - 1075 + top + 127;
-  if (elo > 0) r.lo = __uint_as_float(sign | ((unsigned)elo << 23) | frac);
-  return r;
+  const int r = max(1, 5 - __clzll(top));   // 1..3 for an orthonormal Q
+  const long long half = 1LL << (r - 1);
+#pragma unroll
+  for (int n = NODE0 ? 0 : 1; n < 4; n++)
+#pragma unroll
+    for (int i = 0; i < 3; i++) sa[3 * n + i][threadIdx.x] = fx_split((x[n][i] + half) >> r);
+  return E + 1 + r;
 }
 
-// exact float -> double by bit operations (zero and subnormal floats give 0)
-__device__ __forceinline__ double df_widen(float f) {
-  const unsigned u = __float_as_uint(f);
-  const unsigned long long sign = (unsigned long long)(u & 0x80000000u) << 32;
-  const unsigned ef = (u >> 23) & 0xFFu;
-  if (ef == 0) return __longlong_as_double((long long)sign);
-  const unsigned long long e = ef == 255 ? 0x7FFull : (unsigned long long)(ef - 127 + 1023);
-  return __longlong_as_double((long long)(sign | (e << 52) | ((unsigned long long)(u & 0x7FFFFFu) << 29)));
+__device__ __forceinline__ void fx_digits9(const double (&v)[9], int E, int2 (&d)[9]) {
+#pragma unroll
+  for (int i = 0; i < 9; i++) d[i] = fx_digits(v[i], E);
 }
 
-__device__ __forceinline__ double df_value(DFv a) { return df_widen(a.hi) + df_widen(a.lo); }
-
-__device__ __forceinline__ DFv df_mul(DFv a, DFv b) {
-  const float p = a.hi * b.hi;
-  float e = fmaf(a.hi, b.hi, -p);   // a.hi b.hi = p + e exactly
-  e = fmaf(a.hi, b.lo, e);
-  e = fmaf(a.lo, b.hi, e);
-  const float s = p + e;
-  return DFv{s, e - (s - p)};
+// f_n = V Q sigma g_n (n > 0) and f_0 = -(f_1 + f_2 + f_3), Q orthonormal.  In
+// FP64: in fixed point these 70 operations made the kernels 5% slower, the
+// FP64 units being half idle beside the stiffness.
+template <int MODE>
+__device__ __forceinline__ void stress_forces(const double (&Q)[9], const double (&st)[9], const double (&Di)[9], double vol,
+                                              const ElemOut<MODE>& out) {
+  double P[9], f[12];
+#pragma unroll
+  for (int i = 0; i < 3; i++)
+#pragma unroll
+    for (int j = 0; j < 3; j++)
+      P[i * 3 + j] = (Q[i * 3] * st[j] + Q[i * 3 + 1] * st[3 + j] + Q[i * 3 + 2] * st[6 + j]) * vol;
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    f[i] = 0.0;
+#pragma unroll
+    for (int n = 0; n < 3; n++) {
+      f[3 * (n + 1) + i] = P[i * 3] * Di[n * 3] + P[i * 3 + 1] * Di[n * 3 + 1] + P[i * 3 + 2] * Di[n * 3 + 2];
+      f[i] -= f[3 * (n + 1) + i];
+    }
+  }
+  out.forces(f);
 }
 
-__device__ __forceinline__ DFv df_add(DFv a, DFv b) {
-  const float s = a.hi + b.hi;
-  const float v = s - a.hi;
-  const float t = (a.hi - (s - v)) + (b.hi - v);   // a.hi + b.hi = s + t exactly
-  const float lo = (t + a.lo) + b.lo;
-  const float r = s + lo;
-  return DFv{r, lo - (r - s)};
+// The corotational stiffness R K0_ab R^T = V (lambda h_a h_b^T + mu h_b h_a^T +
+// mu (h_a . h_b) I), h = R g: K0 is isotropic, so rotating it is rotating the
+// gradients (tetelement.cpp:501-544, 583-651).
+template <int MODE>
+__device__ __noinline__ void corot_stiffness64(const double* R, const double* Di, double lv, double mv, ElemOut<MODE> out) {
+  double h[4][3];
+  for (int i = 0; i < 3; i++) {
+    h[0][i] = 0.0;
+    for (int n = 0; n < 3; n++) {
+      h[n + 1][i] = R[i * 3] * Di[n * 3] + R[i * 3 + 1] * Di[n * 3 + 1] + R[i * 3 + 2] * Di[n * 3 + 2];
+      h[0][i] -= h[n + 1][i];
+    }
+  }
+  for (int a = 0; a < 4; a++)
+    for (int b = a; b < 4; b++) {
+      const double dot = mv * (h[a][0] * h[b][0] + h[a][1] * h[b][1] + h[a][2] * h[b][2]);
+      double o[9];
+      for (int i = 0; i < 3; i++)
+        for (int j = 0; j < 3; j++) o[i * 3 + j] = lv * h[a][i] * h[b][j] + mv * h[b][i] * h[a][j] + (i == j ? dot : 0.0);
+      out.block(a, b, o);
+    }
+}
+
+template <int MODE>
+__device__ __forceinline__ void corot_stiffness(const double (&R)[9], const double (&Di)[9], double lv, double mv,
+                                                int2 (*sa)[kElThreads], const ElemOut<MODE>& out) {
+  const int eD = max_exp(Di), eL = max(fx_biased_exp(lv), fx_biased_exp(mv));
+  if (!(max_exp(R) <= 1023 && exp_fits(eD) && exp_fits(eL))) {
+    corot_stiffness64<MODE>(R, Di, lv, mv, out);
+    return;
+  }
+  int2 dR[9], dD[9];
+  fx_digits9(R, 1, dR);
+  fx_digits9(Di, eD - 1022, dD);
+  const int Ea = fx_gradients<true>(dR, dD, eD - 1022, sa), El = eL - 1022;
+  const int2 dl = fx_digits(lv, El), dm = fx_digits(mv, El);
+#pragma unroll 1
+  for (int a = 0; a < 4; a++) {
+    // V lambda h_a and V mu h_a at the scale El + Ea: one place spare, five
+    // products of a diagonal value in one sum
+    int2 ha[3], la[3], ma[3];
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      ha[i] = sa[3 * a + i][threadIdx.x];
+      FxAcc c, d;
+      c.add(dl, ha[i]);
+      d.add(dm, ha[i]);
+      la[i] = fx_norm(c, 2);
+      ma[i] = fx_norm(d, 2);
+    }
+#pragma unroll 1
+    for (int b = a; b < 4; b++) {
+      int2 hb[3];
+#pragma unroll
+      for (int i = 0; i < 3; i++) hb[i] = sa[3 * b + i][threadIdx.x];
+      FxAcc dot;
+#pragma unroll
+      for (int i = 0; i < 3; i++) dot.add(ma[i], hb[i]);
+      double o[9];
+#pragma unroll
+      for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+          FxAcc c;
+          if (i == j) c = dot;
+          c.add(la[i], hb[j]);
+          c.add(ma[j], hb[i]);
+          o[i * 3 + j] = fx_out(c, El + 2 * Ea);
+        }
+      out.block(a, b, o);
+    }
+  }
 }
 
 // -------------------------------------------------- corotational element
 // F = [x1-x0, x2-x0, x3-x0] Dm^-1; R = polar(F), or the proper QR factor when
 // the deformed volume is below threshold * rest volume
-// (tetelement.cpp:546-573); K_ab = R K0_ab R^T packed into 78 values and
-// f_a = sum_b (R K0_ab R^T x_b - R K0_ab X_b) (tetelement.cpp:583-651).
-// MODE 0 scatters into K / fint through the element map (one colour per
-// launch); MODE 1 stores per-element values in original element order;
-// MODE 2 stores them in the colour-ordered staging arrays (all elements in
-// one launch, scattered afterwards colour by colour).
-template <int MODE, bool DF = false>
-__device__ __forceinline__ void corot_elem(int e, int ne, const int4* __restrict__ tets,
-                                           const double* __restrict__ X, const double* __restrict__ u,
-                                           const double* __restrict__ pre, double thr,
-                                           const int* __restrict__ emap, const int* __restrict__ gdof,
-                                           double* __restrict__ K, double* __restrict__ fint,
-                                           double* __restrict__ out78, double* __restrict__ out12,
-                                           const int* __restrict__ perm) {
-  int4 t = tets[e];
-  const int nd[4] = {t.x, t.y, t.z, t.w};
-  V3t<double> o[4], c[4];
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    o[i] = ld3(X, nd[i]);
-    V3t<double> du = ld3(u, nd[i]);
-    c[i] = {o[i].x + du.x, o[i].y + du.y, o[i].z + du.z};
-  }
-  double Di[9], F[9];
-#pragma unroll
-  for (int i = 0; i < 9; i++) { Di[i] = pre[(size_t)(90 + i) * ne + e]; F[i] = 0.0; }
-#pragma unroll
-  for (int i = 1; i < 4; i++) {
-    double ax[3] = {c[i].x - c[0].x, c[i].y - c[0].y, c[i].z - c[0].z};
-#pragma unroll
-    for (int j = 0; j < 3; j++)
-#pragma unroll
-      for (int k = 0; k < 3; k++) F[j * 3 + k] += ax[j] * Di[(i - 1) * 3 + k];
-  }
-  const double v0 = pre[(size_t)99 * ne + e];
-  const double v1 = tet_vol(c[0], c[1], c[2], c[3]);
-  double R[9];
-  if (v1 >= thr * v0) polar3<double>(F, R);
-  else qr3<double>(F, R);
-
-  double f[12];
-#pragma unroll
-  for (int i = 0; i < 12; i++) f[i] = 0.0;
-  const size_t obase = MODE == 1 ? (size_t)perm[e] * 78 : 0;
-  auto put = [&](int k, double val) {
-    if (MODE == 0) {
-      int idx = emap[(size_t)k * ne + e];
-      if (idx >= 0) K[idx] += val;
-    } else if (MODE == 1) {
-      out78[obase + k] = val;
-    } else {
-      out78[kst(k, e)] = val;
-    }
-  };
-  if constexpr (DF) {
-    // The mixed-precision path: forces f_a = R sum_b K0_ab (R^T c_b - o_b) in
-    // FP64 (the same sum regrouped, the cancellation of R^T c_b against o_b
-    // taken first) and the stiffness R K0_ab R^T in double-float.
-    double y[4][3], g[4][3];
-#pragma unroll
-    for (int b = 0; b < 4; b++) {
-      const double cb[3] = {c[b].x, c[b].y, c[b].z}, ob[3] = {o[b].x, o[b].y, o[b].z};
-#pragma unroll
-      for (int i = 0; i < 3; i++) {
-        y[b][i] = (R[i] * cb[0] + R[3 + i] * cb[1] + R[6 + i] * cb[2]) - ob[i];
-        g[b][i] = 0.0;
-      }
-    }
-    DFv dR[9];
-#pragma unroll
-    for (int i = 0; i < 9; i++) dR[i] = df_split(R[i]);
-    int blk = 0;
-#pragma unroll 1
-    for (int a = 0; a < 4; a++) {
-#pragma unroll 1
-      for (int b = a; b < 4; b++) {
-        double K0[9];
-#pragma unroll
-        for (int i = 0; i < 9; i++) K0[i] = pre[(size_t)(9 * blk + i) * ne + e];
-        blk++;
-#pragma unroll
-        for (int i = 0; i < 3; i++) {
-          g[a][i] += K0[i * 3] * y[b][0] + K0[i * 3 + 1] * y[b][1] + K0[i * 3 + 2] * y[b][2];
-          if (b != a) g[b][i] += K0[i] * y[a][0] + K0[3 + i] * y[a][1] + K0[6 + i] * y[a][2];
-        }
-        DFv dQK[9];
-#pragma unroll
-        for (int i = 0; i < 3; i++)
-#pragma unroll
-          for (int j = 0; j < 3; j++)
-            dQK[i * 3 + j] = df_add(df_add(df_mul(dR[i * 3], df_split(K0[j])), df_mul(dR[i * 3 + 1], df_split(K0[3 + j]))),
-                                    df_mul(dR[i * 3 + 2], df_split(K0[6 + j])));
-        auto qkqt = [&](int i, int j) {
-          return df_value(df_add(df_add(df_mul(dQK[i * 3], dR[j * 3]), df_mul(dQK[i * 3 + 1], dR[j * 3 + 1])),
-                                 df_mul(dQK[i * 3 + 2], dR[j * 3 + 2])));
-        };
-        if (a == b) {
-#pragma unroll
-          for (int i = 0; i < 3; i++)
-#pragma unroll
-            for (int j = 0; j < 3 - i; j++) put(c_diag12[a * 3 + i] + j, qkqt(i, i + j));
-        } else {
-#pragma unroll
-          for (int i = 0; i < 3; i++)
-#pragma unroll
-            for (int j = 0; j < 3; j++) put(c_diag12[a * 3 + i] + (b - a) * 3 - i + j, qkqt(i, j));
-        }
-      }
-    }
-#pragma unroll
-    for (int a = 0; a < 4; a++)
-#pragma unroll
-      for (int i = 0; i < 3; i++) f[a * 3 + i] = R[i * 3] * g[a][0] + R[i * 3 + 1] * g[a][1] + R[i * 3 + 2] * g[a][2];
-  } else {
-  int blk = 0;
-#pragma unroll 1
-  for (int a = 0; a < 4; a++) {
-    double K0[9], QK[9], QKQT[9];
-#pragma unroll
-    for (int i = 0; i < 9; i++) K0[i] = pre[(size_t)(9 * blk + i) * ne + e];
-    blk++;
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-      for (int j = 0; j < 3; j++) QK[i * 3 + j] = R[i * 3] * K0[j] + R[i * 3 + 1] * K0[3 + j] + R[i * 3 + 2] * K0[6 + j];
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-      for (int j = 0; j < 3; j++) QKQT[i * 3 + j] = QK[i * 3] * R[j * 3] + QK[i * 3 + 1] * R[j * 3 + 1] + QK[i * 3 + 2] * R[j * 3 + 2];
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-      for (int j = 0; j < 3 - i; j++) put(c_diag12[a * 3 + i] + j, QKQT[i * 3 + i + j]);
-    const double ca[3] = {c[a].x, c[a].y, c[a].z}, oa[3] = {o[a].x, o[a].y, o[a].z};
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-      for (int j = 0; j < 3; j++) f[a * 3 + i] += QKQT[i * 3 + j] * ca[j] - QK[i * 3 + j] * oa[j];
-#pragma unroll 1
-    for (int b = a + 1; b < 4; b++) {
-      double QKT[9];
-#pragma unroll
-      for (int i = 0; i < 9; i++) K0[i] = pre[(size_t)(9 * blk + i) * ne + e];
-      blk++;
-#pragma unroll
-      for (int i = 0; i < 3; i++)
-#pragma unroll
-        for (int j = 0; j < 3; j++) {
-          QK[i * 3 + j] = R[i * 3] * K0[j] + R[i * 3 + 1] * K0[3 + j] + R[i * 3 + 2] * K0[6 + j];
-          QKT[i * 3 + j] = R[i * 3] * K0[j * 3] + R[i * 3 + 1] * K0[j * 3 + 1] + R[i * 3 + 2] * K0[j * 3 + 2];
-        }
-#pragma unroll
-      for (int i = 0; i < 3; i++)
-#pragma unroll
-        for (int j = 0; j < 3; j++) QKQT[i * 3 + j] = QK[i * 3] * R[j * 3] + QK[i * 3 + 1] * R[j * 3 + 1] + QK[i * 3 + 2] * R[j * 3 + 2];
-      const double cb[3] = {c[b].x, c[b].y, c[b].z}, ob[3] = {o[b].x, o[b].y, o[b].z};
-#pragma unroll
-      for (int i = 0; i < 3; i++)
-#pragma unroll
-        for (int j = 0; j < 3; j++) {
-          put(c_diag12[a * 3 + i] + (b - a) * 3 - i + j, QKQT[i * 3 + j]);
-          f[a * 3 + i] += QKQT[i * 3 + j] * cb[j] - QK[i * 3 + j] * ob[j];
-          f[b * 3 + i] += QKQT[j * 3 + i] * ca[j] - QKT[i * 3 + j] * oa[j];
-        }
-    }
-  }
-  }
-  if (MODE == 0) {
-#pragma unroll
-    for (int k = 0; k < 12; k++) {
-      int g = gdof[(size_t)k * ne + e];
-      if (g >= 0) fint[g] += f[k];
-    }
-  } else if (MODE == 1) {
-#pragma unroll
-    for (int k = 0; k < 12; k++) out12[(size_t)perm[e] * 12 + k] = f[k];
-  } else {
-#pragma unroll
-    for (int k = 0; k < 12; k++) out12[fst(k, e)] = f[k];
-  }
-}
-
-// ------------------------------------------- invertible hyperelastic element
-// Invertible SVD of F, energy derivatives in the invariants I1 = sum s^2,
-// I2 = sum s^4, I3 = prod s^2 (invertibleHyperelastic.h:22-30): Neo-Hookean
-// (invertibleNeoHookean.cpp:11-20) or StVK (invertibleStVK.cpp:11-20);
-// P = U diag(2 g1 s + 4 g2 s^3 + 2 g3 I3 / s) V^T (invertibleHyperelastic.cpp:
-// 247-265); dP/dF in the singular-value frame projected to PSD
-// (tetelement.cpp:357-499) -- only its 21 structural non-zeros are formed;
-// K_ab = U [sum_kl dP_ikjl (V^T dN_a)_k (V^T dN_b)_l] U^T / (36 V)
-// (tetelement.cpp:282-342); f_a = P dN_a / 6, f_3 = -(f_0 + f_1 + f_2)
-// (tetelement.cpp:344-355).
-template <int MODE, bool DF = false>
-__device__ __forceinline__ void invhyper_elem(int e, int ne, int stvk, const int4* __restrict__ tets,
-                                              const double* __restrict__ X, const double* __restrict__ u,
-                                              const double* __restrict__ pre, double thr, double lambda, double mu,
-                                              const int* __restrict__ emap, const int* __restrict__ gdof,
-                                              double* __restrict__ K, double* __restrict__ fint,
-                                              double* __restrict__ out78, double* __restrict__ out12,
-                                              const int* __restrict__ perm) {
+// (tetelement.cpp:546-573); S = R^T F.
+__device__ __forceinline__ void corot_frame(int e, int ne, const int4* __restrict__ tets, const double* __restrict__ X,
+                                            const double* __restrict__ u, const double* __restrict__ pre, double thr,
+                                            double (&Di)[9], double& v0, double (&R)[9], double (&S)[9]) {
   int4 t = tets[e];
   const int nd[4] = {t.x, t.y, t.z, t.w};
   V3t<double> c[4];
@@ -458,31 +383,254 @@ __device__ __forceinline__ void invhyper_elem(int e, int ne, int stvk, const int
   }
   double F[9];
 #pragma unroll
-  for (int i = 0; i < 9; i++) F[i] = 0.0;
+  for (int i = 0; i < 9; i++) { Di[i] = pre[(size_t)i * ne + e]; F[i] = 0.0; }
 #pragma unroll
   for (int i = 1; i < 4; i++) {
     double ax[3] = {c[i].x - c[0].x, c[i].y - c[0].y, c[i].z - c[0].z};
 #pragma unroll
     for (int j = 0; j < 3; j++)
 #pragma unroll
-      for (int k = 0; k < 3; k++) F[j * 3 + k] += ax[j] * pre[(size_t)(12 + (i - 1) * 3 + k) * ne + e];
+      for (int k = 0; k < 3; k++) F[j * 3 + k] += ax[j] * Di[(i - 1) * 3 + k];
+  }
+  v0 = pre[(size_t)kPreVol * ne + e];
+  const double v1 = tet_vol(c[0], c[1], c[2], c[3]);
+  if (v1 >= thr * v0) polar3<double>(F, R);
+  else qr3<double>(F, R);
+#pragma unroll
+  for (int i = 0; i < 3; i++)
+#pragma unroll
+    for (int j = 0; j < 3; j++) S[i * 3 + j] = R[i] * F[j] + R[3 + i] * F[3 + j] + R[6 + i] * F[6 + j];
+}
+
+// Corotational linear element: f_a = sum_b (R K0_ab R^T x_b - R K0_ab X_b)
+// (tetelement.cpp:583-651), which for the isotropic K0 is the stress of the
+// strain sym(S) - I on the rotated gradients; K_ab = R K0_ab R^T.
+template <int MODE>
+__device__ __forceinline__ void corot_elem(int e, int ne, const int4* __restrict__ tets, const double* __restrict__ X,
+                                           const double* __restrict__ u, const double* __restrict__ pre, double thr,
+                                           double lambda, double mu, double* __restrict__ out78,
+                                           double* __restrict__ out12, const int* __restrict__ perm,
+                                           int2 (*sa)[kElThreads]) {
+  double Di[9], R[9], S[9], v0, st[9];
+  corot_frame(e, ne, tets, X, u, pre, thr, Di, v0, R, S);
+  const ElemOut<MODE> out(e, out78, out12, perm);
+  const double d0 = S[0] - 1.0, d1 = S[4] - 1.0, d2 = S[8] - 1.0, dg = lambda * (d0 + d1 + d2), mu2 = 2.0 * mu;
+  st[0] = mu2 * d0 + dg;
+  st[4] = mu2 * d1 + dg;
+  st[8] = mu2 * d2 + dg;
+  st[1] = st[3] = mu * (S[1] + S[3]);
+  st[2] = st[6] = mu * (S[2] + S[6]);
+  st[5] = st[7] = mu * (S[5] + S[7]);
+  stress_forces<MODE>(R, st, Di, v0, out);
+  corot_stiffness<MODE>(R, Di, lambda * v0, mu * v0, sa, out);
+}
+
+// ------------------------------------------- invertible hyperelastic element
+// K_ab = V U [sum_kl dP_ikjl a_ak a_bl] U^T, a_n = V^T g_n (tetelement.cpp:282-342),
+// dP/dF in the singular frame by its 21 structural non-zeros: T (the
+// diagonal's), Al and Be (tetelement.cpp:357-499).
+template <int MODE>
+__device__ __noinline__ void hyper_stiffness64(const double* U, const double* VT, const double* Di, const double* T6,
+                                               const double* al, const double* be, double vol, ElemOut<MODE> out) {
+  double an[4][3], T[3][3] = {{T6[0], T6[1], T6[2]}, {T6[1], T6[3], T6[4]}, {T6[2], T6[4], T6[5]}};
+  for (int i = 0; i < 3; i++) {
+    an[0][i] = 0.0;
+    for (int n = 0; n < 3; n++) {
+      an[n + 1][i] = VT[i * 3] * Di[n * 3] + VT[i * 3 + 1] * Di[n * 3 + 1] + VT[i * 3 + 2] * Di[n * 3 + 2];
+      an[0][i] -= an[n + 1][i];
+    }
+  }
+  for (int a = 0; a < 4; a++)
+    for (int b = a; b < 4; b++) {
+      double sm[9], tmp[9], o[9];
+      for (int i = 0; i < 3; i++)
+        for (int j = 0; j < 3; j++) {
+          double en = 0.0;
+          if (i == j) {
+            for (int k = 0; k < 3; k++) en += (k == i ? T[i][i] : al[i + k - 1]) * an[a][k] * an[b][k];
+          } else {
+            en = T[i][j] * an[a][i] * an[b][j] + be[i + j - 1] * an[a][j] * an[b][i];
+          }
+          sm[i * 3 + j] = en;
+        }
+      mul3(U, sm, tmp);
+      for (int i = 0; i < 3; i++)
+        for (int j = 0; j < 3; j++)
+          o[i * 3 + j] = (tmp[i * 3] * U[j * 3] + tmp[i * 3 + 1] * U[j * 3 + 1] + tmp[i * 3 + 2] * U[j * 3 + 2]) * vol;
+      out.block(a, b, o);
+    }
+}
+
+// al, be: entries (0,1), (0,2), (1,2); the index of (i, k) is i + k - 1
+template <int MODE>
+__device__ __forceinline__ void hyper_stiffness(const double (&U)[9], const double (&VT)[9], const double (&Di)[9],
+                                                const double (&T6)[6], const double (&al)[3], const double (&be)[3],
+                                                double vol, HyperShared& sh, const ElemOut<MODE>& out) {
+  const int eT = max_exp(T6, max_exp(al, max_exp(be))), eD = max_exp(Di), eV = fx_biased_exp(vol);
+  if (!(max_exp(U, max_exp(VT)) <= 1023 && exp_fits(eT) && exp_fits(eD) && exp_fits(eV))) {
+    hyper_stiffness64<MODE>(U, VT, Di, T6, al, be, vol, out);
+    return;
+  }
+  const int2 dv = fx_digits(vol, eV - 1022);
+  int2 dU[9], dD[9], dVT[9];
+  fx_digits9(U, 1, dU);
+  fx_digits9(Di, eD - 1022, dD);
+  fx_digits9(VT, 1, dVT);
+  const int Ea = fx_gradients<false>(dVT, dD, eD - 1022, sh.g);
+  // V dP/dF at the scale Et
+  auto times_vol = [&](double t) {
+    FxAcc c;
+    c.add(fx_digits(t, eT - 1022), dv);
+    return fx_norm(c, 2);
+  };
+  int2 dT[6], dA[3], dB[3];
+#pragma unroll
+  for (int i = 0; i < 6; i++) dT[i] = times_vol(T6[i]);
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    dA[i] = times_vol(al[i]);
+    dB[i] = times_vol(be[i]);
+  }
+  auto sym6 = [](int i, int j) { return i <= j ? i * 3 - (i * (i - 1)) / 2 + (j - i) : j * 3 - (j * (j - 1)) / 2 + (i - j); };
+  const int Et = eT + eV - 2044;
+  // Blocks of nodes 1..3 by products; a column of blocks sums to zero (the
+  // gradients do), so node 0's follow by exact integer sums.
+  const int Ek = Et + 2 * Ea + 2;
+#pragma unroll
+  for (int i = 0; i < 27; i++) sh.row0[i][threadIdx.x] = 0;
+#pragma unroll 1
+  for (int a = 1; a < 4; a++) {
+    // dP/dF contracted with node a's gradient, at the scale Et + Ea - 1
+    int2 ha[3], wd[3][3], wo[3][3], wb[3][3];   // diagonal values' terms by k; T_ij a_i; Be_ij a_j
+#pragma unroll
+    for (int i = 0; i < 3; i++) ha[i] = sh.g[3 * a + i][threadIdx.x];
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+      for (int j = 0; j < 3; j++) {
+        auto times = [&](int2 t, int2 h) {
+          FxAcc c;
+          c.add(t, h);
+          return fx_norm(c, 1);
+        };
+        wd[i][j] = times(i == j ? dT[sym6(i, i)] : dA[i + j - 1], ha[j]);
+        if (i != j) {
+          wo[i][j] = times(dT[sym6(i, j)], ha[i]);
+          wb[i][j] = times(dB[i + j - 1], ha[j]);
+        }
+      }
+#pragma unroll 1
+    for (int b = a; b < 4; b++) {
+      int2 hb[3], sm[9], tmp[9];
+#pragma unroll
+      for (int i = 0; i < 3; i++) hb[i] = sh.g[3 * b + i][threadIdx.x];
+      // at the scale Et + 2 Ea: three products, below 0.75 of it
+#pragma unroll
+      for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+          FxAcc c;
+          if (i == j) {
+#pragma unroll
+            for (int k = 0; k < 3; k++) c.add(wd[i][k], hb[k]);
+          } else {
+            c.add(wo[i][j], hb[j]);
+            c.add(wb[i][j], hb[i]);
+          }
+          sm[i * 3 + j] = fx_norm(c, 3);
+        }
+      // U sm, at the scale Et + 2 Ea + 1
+#pragma unroll
+      for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+          FxAcc c;
+#pragma unroll
+          for (int k = 0; k < 3; k++) c.add(sm[k * 3 + j], dU[i * 3 + k]);
+          tmp[i * 3 + j] = fx_norm(c, 2);
+        }
+      // (U sm) U^T: below 0.57 2^62 in units of 2^(Ek - 62), so three of them
+      // fit an integer
+      double o[9];
+#pragma unroll
+      for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+          FxAcc c;
+#pragma unroll
+          for (int k = 0; k < 3; k++) c.add(tmp[i * 3 + k], dU[j * 3 + k]);
+          const long long x = c.hh + (c.mid >> kFxLow);
+          sh.row0[9 * (b - 1) + 3 * i + j][threadIdx.x] -= x;
+          if (a != b) sh.row0[9 * (a - 1) + 3 * j + i][threadIdx.x] -= x;
+          o[i * 3 + j] = fx_double(x, Ek - 2 * (kFxBits - kFxLow));
+        }
+      out.block(a, b, o);
+    }
+  }
+  long long own[9];
+#pragma unroll
+  for (int i = 0; i < 9; i++) own[i] = 0;
+#pragma unroll 1
+  for (int b = 1; b < 4; b++) {
+    double o[9];
+#pragma unroll
+    for (int i = 0; i < 9; i++) {
+      const long long x = sh.row0[9 * (b - 1) + i][threadIdx.x];
+      own[i] -= x >> 2;
+      o[i] = fx_double(x, Ek - 2 * (kFxBits - kFxLow));
+    }
+    out.block(0, b, o);
+  }
+  double o[9];
+#pragma unroll
+  for (int i = 0; i < 9; i++) o[i] = fx_double(own[i], Ek + 2 - 2 * (kFxBits - kFxLow));
+  out.block(0, 0, o);
+}
+
+// Invertible SVD of F, energy derivatives in the invariants I1 = sum s^2,
+// I2 = sum s^4, I3 = prod s^2 (invertibleHyperelastic.h:22-30): Neo-Hookean
+// (invertibleNeoHookean.cpp:11-20) or StVK (invertibleStVK.cpp:11-20);
+// P = U diag(2 g1 s + 4 g2 s^3 + 2 g3 I3 / s) V^T (invertibleHyperelastic.cpp:
+// 247-265); dP/dF in the singular-value frame projected to PSD
+// (tetelement.cpp:357-499); f_n = V P g_n, f_0 = -(f_1 + f_2 + f_3)
+// (tetelement.cpp:344-355).  I3 / s_i and I3 / (s_i s_j) are the products of
+// the other factors: FP64 divisions are long instruction sequences.
+template <int MODE>
+__device__ __forceinline__ void invhyper_elem(int e, int ne, int stvk, const int4* __restrict__ tets,
+                                              const double* __restrict__ X, const double* __restrict__ u,
+                                              const double* __restrict__ pre, double thr, double lambda, double mu,
+                                              double* __restrict__ out78, double* __restrict__ out12,
+                                              const int* __restrict__ perm, HyperShared& sh) {
+  int4 t = tets[e];
+  const int nd[4] = {t.x, t.y, t.z, t.w};
+  V3t<double> c[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    V3t<double> x = ld3(X, nd[i]), du = ld3(u, nd[i]);
+    c[i] = {x.x + du.x, x.y + du.y, x.z + du.z};
+  }
+  double F[9], Di[9];
+#pragma unroll
+  for (int i = 0; i < 9; i++) { Di[i] = pre[(size_t)i * ne + e]; F[i] = 0.0; }
+#pragma unroll
+  for (int i = 1; i < 4; i++) {
+    double ax[3] = {c[i].x - c[0].x, c[i].y - c[0].y, c[i].z - c[0].z};
+#pragma unroll
+    for (int j = 0; j < 3; j++)
+#pragma unroll
+      for (int k = 0; k < 3; k++) F[j * 3 + k] += ax[j] * Di[(i - 1) * 3 + k];
   }
   double sig[3], U[9], VT[9];
-  invertible_svd<double, DF>(F, thr, sig, U, VT);
+  invertible_svd<double, true>(F, thr, sig, U, VT);
   const double s02 = sig[0] * sig[0], s12 = sig[1] * sig[1], s22 = sig[2] * sig[2];
   const double I1 = s02 + s12 + s22, I3 = s02 * s12 * s22;
   double g0, g1, g2, h0 = 0.0, h5 = 0.0;
   if (!stvk) {
+    const double lI3 = log(I3), rI3 = 1.0 / I3;
     g0 = 0.5 * mu;
     g1 = 0.0;
-    if constexpr (DF) {   // one reciprocal of I3 for both
-      const double lI3 = log(I3), rI3 = 1.0 / I3;
-      g2 = (-0.5 * mu + 0.25 * lambda * lI3) * rI3;
-      h5 = (0.5 * mu + 0.25 * lambda * (1.0 - lI3)) * (rI3 * rI3);
-    } else {
-      g2 = (-0.5 * mu + 0.25 * lambda * log(I3)) / I3;
-      h5 = (0.5 * mu + 0.25 * lambda * (1.0 - log(I3))) / (I3 * I3);
-    }
+    g2 = (-0.5 * mu + 0.25 * lambda * lI3) * rI3;
+    h5 = (0.5 * mu + 0.25 * lambda * (1.0 - lI3)) * (rI3 * rI3);
   } else {
     g0 = 0.25 * lambda * (I1 - 3.0) - 0.5 * mu;
     g1 = 0.25 * mu;
@@ -491,260 +639,83 @@ __device__ __forceinline__ void invhyper_elem(int e, int ne, int stvk, const int
   }
   // dP/dF non-zeros (tetelement.cpp:357-437)
   const double sc01 = sig[0] * sig[1], sc02 = sig[0] * sig[2], sc12 = sig[1] * sig[2];
-  double a01 = 2.0 * g0 + 4.0 * (s02 + s12) * g1;
-  double a02 = 2.0 * g0 + 4.0 * (s02 + s22) * g1;
-  double a12 = 2.0 * g0 + 4.0 * (s12 + s22) * g1;
+  double al[3] = {2.0 * g0 + 4.0 * (s02 + s12) * g1, 2.0 * g0 + 4.0 * (s02 + s22) * g1,
+                  2.0 * g0 + 4.0 * (s12 + s22) * g1};
   const double a00 = 2.0 * g0 + 8.0 * s02 * g1, a11 = 2.0 * g0 + 8.0 * s12 * g1, a22 = 2.0 * g0 + 8.0 * s22 * g1;
-  // d_ij = I3 g2 / (s_i s_j); the mixed path forms them as products
-  // (I3 / (s_i s_j) is the product of the other factors: FP64 divisions are
-  // long instruction sequences on this part), and so its forces' I3 / s_i;
-  // the FP64 path keeps the reference's expressions.
-  const double d00 = DF ? g2 * (s12 * s22) : I3 * g2 / s02, d01 = DF ? g2 * (sc01 * s22) : I3 * g2 / sc01,
-               d02 = DF ? g2 * (sc02 * s12) : I3 * g2 / sc02;
-  const double d11 = DF ? g2 * (s02 * s22) : I3 * g2 / s12, d12 = DF ? g2 * (sc12 * s02) : I3 * g2 / sc12,
-               d22 = DF ? g2 * (s02 * s12) : I3 * g2 / s22;
+  // d_ij = I3 g2 / (s_i s_j)
+  const double d00 = g2 * (s12 * s22), d01 = g2 * (sc01 * s22), d02 = g2 * (sc02 * s12);
+  const double d11 = g2 * (s02 * s22), d12 = g2 * (sc12 * s02), d22 = g2 * (s02 * s12);
   const double b00 = 4.0 * s02 * g1 - 2.0 * d00, b11 = 4.0 * s12 * g1 - 2.0 * d11, b22 = 4.0 * s22 * g1 - 2.0 * d22;
-  double b01 = 4.0 * sc01 * g1 - 2.0 * d01, b02 = 4.0 * sc02 * g1 - 2.0 * d02, b12 = 4.0 * sc12 * g1 - 2.0 * d12;
-  // Hessian in the invariants is diag-like: only H00 (StVK) or H22 (NH) set
-  double w[3][3];
-#pragma unroll
-  for (int i = 0; i < 3; i++) {
-    w[i][0] = 2.0 * sig[i];
-    w[i][1] = 4.0 * sig[i] * (i == 0 ? s02 : (i == 1 ? s12 : s22));
-    w[i][2] = DF ? 2.0 * sig[i] * (i == 0 ? s12 * s22 : (i == 1 ? s02 * s22 : s02 * s12)) : 2.0 * I3 / sig[i];
-  }
-  // w_i . (H w_j) with H = diag(h0, 0, h5) in the invariants (the only
-  // non-zero Hessian entries of both energies)
-  auto qf = [&](int i, int j) { return w[i][0] * (h0 * w[j][0]) + w[i][2] * (h5 * w[j][2]); };
+  double be[3] = {4.0 * sc01 * g1 - 2.0 * d01, 4.0 * sc02 * g1 - 2.0 * d02, 4.0 * sc12 * g1 - 2.0 * d12};
+  // I3 / s_i, and the rows of the invariants' derivatives the Hessians touch:
+  // only H00 (StVK) or H22 (Neo-Hookean) is set
+  const double q0 = sig[0] * (s12 * s22), q1 = sig[1] * (s02 * s22), q2 = sig[2] * (s02 * s12);
+  const double w0[3] = {2.0 * sig[0], 2.0 * sig[1], 2.0 * sig[2]}, w2[3] = {2.0 * q0, 2.0 * q1, 2.0 * q2};
+  auto qf = [&](int i, int j) { return w0[i] * (h0 * w0[j]) + w2[i] * (h5 * w2[j]); };
   double T[6] = {a00 + b00 + (qf(0, 0) + 4.0 * d00), qf(1, 0) + 4.0 * d01, qf(2, 0) + 4.0 * d02,
                  a11 + b11 + (qf(1, 1) + 4.0 * d11), qf(2, 1) + 4.0 * d12, a22 + b22 + (qf(2, 2) + 4.0 * d22)};
   psd3<double>(T);
-  psd2<double>(a01, b01);
-  psd2<double>(a02, b02);
-  psd2<double>(a12, b12);
-  const double Tm[3][3] = {{T[0], T[1], T[2]}, {T[1], T[3], T[4]}, {T[2], T[4], T[5]}};
-  const double Al[3][3] = {{0.0, a01, a02}, {a01, 0.0, a12}, {a02, a12, 0.0}};
-  const double Be[3][3] = {{0.0, b01, b02}, {b01, 0.0, b12}, {b02, b12, 0.0}};
-
-  // P = U diag(de) V^T
-  double de[3], P[9];
+#pragma unroll
+  for (int i = 0; i < 3; i++) psd2<double>(al[i], be[i]);
+  const double vol = pre[(size_t)kPreVol * ne + e];
+  const ElemOut<MODE> out(e, out78, out12, perm);
+  const double qs[3] = {q0, q1, q2};
+  double dvt[9];
 #pragma unroll
   for (int i = 0; i < 3; i++) {
-    if constexpr (DF) {   // I3 / s_i as the product s_i s_j^2 s_k^2
-      const double i3s = sig[i] * (i == 0 ? s12 * s22 : (i == 1 ? s02 * s22 : s02 * s12));
-      de[i] = 2.0 * g0 * sig[i] + 4.0 * g1 * sig[i] * sig[i] * sig[i] + 2.0 * g2 * i3s;
-    } else {
-      de[i] = 2.0 * g0 * sig[i] + 4.0 * g1 * sig[i] * sig[i] * sig[i] + 2.0 * g2 * I3 / sig[i];
-    }
+    const double de = 2.0 * g0 * sig[i] + 4.0 * g1 * sig[i] * sig[i] * sig[i] + 2.0 * g2 * qs[i];
+#pragma unroll
+    for (int j = 0; j < 3; j++) dvt[i * 3 + j] = de * VT[i * 3 + j];
   }
-#pragma unroll
-  for (int i = 0; i < 3; i++)
-#pragma unroll
-    for (int j = 0; j < 3; j++)
-      P[i * 3 + j] = U[i * 3] * (VT[j] * de[0]) + U[i * 3 + 1] * (VT[3 + j] * de[1]) + U[i * 3 + 2] * (VT[6 + j] * de[2]);
-
-  // a_n = V^T dN_n
-  double an[4][3];
-#pragma unroll
-  for (int nn = 0; nn < 4; nn++) {
-    double d0 = pre[(size_t)(3 * nn) * ne + e], d1 = pre[(size_t)(3 * nn + 1) * ne + e], d2 = pre[(size_t)(3 * nn + 2) * ne + e];
-#pragma unroll
-    for (int i = 0; i < 3; i++) an[nn][i] = VT[3 * i] * d0 + VT[3 * i + 1] * d1 + VT[3 * i + 2] * d2;
-  }
-  const double fac = 1.0 / (36.0 * pre[(size_t)21 * ne + e]);
-  const size_t obase = MODE == 1 ? (size_t)perm[e] * 78 : 0;
-  auto put = [&](int k, double val) {
-    if (MODE == 0) {
-      int idx = emap[(size_t)k * ne + e];
-      if (idx >= 0) K[idx] += val;
-    } else if (MODE == 1) {
-      out78[obase + k] = val;
-    } else {
-      out78[kst(k, e)] = val;
-    }
-  };
-  if constexpr (DF) {
-    // the contraction U [sum_kl dP_ikjl an_a,k an_b,l] U^T / (36 V) in
-    // double-float, the same terms in the same order as below
-    // Tm symmetric (6 values), Al and Be symmetric with zero diagonals (3 each)
-    DFv dan[4][3], dU[9], dT6[6], dA3[3], dB3[3];
-#pragma unroll
-    for (int nn = 0; nn < 4; nn++)
-#pragma unroll
-      for (int i = 0; i < 3; i++) dan[nn][i] = df_split(an[nn][i]);
-#pragma unroll
-    for (int i = 0; i < 9; i++) dU[i] = df_split(U[i]);
-#pragma unroll
-    for (int i = 0; i < 6; i++) dT6[i] = df_split(T[i]);
-    dA3[0] = df_split(a01); dA3[1] = df_split(a02); dA3[2] = df_split(a12);
-    dB3[0] = df_split(b01); dB3[1] = df_split(b02); dB3[2] = df_split(b12);
-    auto sym6 = [](int i, int j) { return i <= j ? i * 3 - (i * (i - 1)) / 2 + (j - i) : j * 3 - (j * (j - 1)) / 2 + (i - j); };
-    auto off3 = [](int i, int j) { return i + j - 1; };   // (0,1) -> 0, (0,2) -> 1, (1,2) -> 2
-    const DFv dfac = df_split(fac);
-#pragma unroll 1
-    for (int a = 0; a < 4; a++) {
-#pragma unroll 1
-      for (int b = a; b < 4; b++) {
-        DFv sm[9];
-#pragma unroll
-        for (int i = 0; i < 3; i++)
-#pragma unroll
-          for (int j = 0; j < 3; j++) {
-            DFv en{0.f, 0.f};
-            if (i == j) {
-#pragma unroll
-              for (int k = 0; k < 3; k++)
-                en = df_add(en, df_mul(df_mul(k == i ? dT6[sym6(i, i)] : dA3[off3(i, k)], dan[a][k]), dan[b][k]));
-            } else if (i < j) {
-              en = df_add(en, df_mul(df_mul(dT6[sym6(i, j)], dan[a][i]), dan[b][j]));
-              en = df_add(en, df_mul(df_mul(dB3[off3(i, j)], dan[a][j]), dan[b][i]));
-            } else {
-              en = df_add(en, df_mul(df_mul(dB3[off3(i, j)], dan[a][j]), dan[b][i]));
-              en = df_add(en, df_mul(df_mul(dT6[sym6(i, j)], dan[a][i]), dan[b][j]));
-            }
-            sm[i * 3 + j] = en;
-          }
-        DFv tmp[9];
-#pragma unroll
-        for (int i = 0; i < 3; i++)
-#pragma unroll
-          for (int j = 0; j < 3; j++)
-            tmp[i * 3 + j] = df_add(df_add(df_mul(dU[i * 3], sm[j]), df_mul(dU[i * 3 + 1], sm[3 + j])),
-                                    df_mul(dU[i * 3 + 2], sm[6 + j]));
-        auto outv = [&](int i, int j) {
-          const DFv o = df_add(df_add(df_mul(tmp[i * 3], dU[j * 3]), df_mul(tmp[i * 3 + 1], dU[j * 3 + 1])),
-                               df_mul(tmp[i * 3 + 2], dU[j * 3 + 2]));
-          return df_value(df_mul(o, dfac));
-        };
-        if (a == b) {
-#pragma unroll
-          for (int i = 0; i < 3; i++)
-#pragma unroll
-            for (int j = 0; j < 3 - i; j++) put(c_diag12[a * 3 + i] + j, outv(i, i + j));
-        } else {
-#pragma unroll
-          for (int i = 0; i < 3; i++)
-#pragma unroll
-            for (int j = 0; j < 3; j++) put(c_diag12[a * 3 + i] + (b - a) * 3 - i + j, outv(i, j));
-        }
-      }
-    }
-  } else {
-#pragma unroll 1
-  for (int a = 0; a < 4; a++) {
-#pragma unroll 1
-    for (int b = a; b < 4; b++) {
-      double sm[9];
-#pragma unroll
-      for (int i = 0; i < 3; i++)
-#pragma unroll
-        for (int j = 0; j < 3; j++) {
-          double en = 0.0;
-          if (i == j) {
-#pragma unroll
-            for (int k = 0; k < 3; k++) en += (k == i ? Tm[i][i] : Al[i][k]) * an[a][k] * an[b][k];
-          } else if (i < j) {
-            en += Tm[i][j] * an[a][i] * an[b][j];
-            en += Be[i][j] * an[a][j] * an[b][i];
-          } else {
-            en += Be[i][j] * an[a][j] * an[b][i];
-            en += Tm[i][j] * an[a][i] * an[b][j];
-          }
-          sm[i * 3 + j] = en;
-        }
-      double tmp[9], out[9];
-      mul3(U, sm, tmp);
-#pragma unroll
-      for (int i = 0; i < 3; i++)
-#pragma unroll
-        for (int j = 0; j < 3; j++) out[i * 3 + j] = tmp[i * 3] * U[j * 3] + tmp[i * 3 + 1] * U[j * 3 + 1] + tmp[i * 3 + 2] * U[j * 3 + 2];
-      if (a == b) {
-#pragma unroll
-        for (int i = 0; i < 3; i++)
-#pragma unroll
-          for (int j = 0; j < 3 - i; j++) put(c_diag12[a * 3 + i] + j, out[i * 3 + i + j] * fac);
-      } else {
-#pragma unroll
-        for (int i = 0; i < 3; i++)
-#pragma unroll
-          for (int j = 0; j < 3; j++) put(c_diag12[a * 3 + i] + (b - a) * 3 - i + j, out[i * 3 + j] * fac);
-      }
-    }
-  }
-  }
-  double f[12];
-  const double sixth = 1.0 / 6.0;
-#pragma unroll
-  for (int nn = 0; nn < 3; nn++) {
-    double d0 = pre[(size_t)(3 * nn) * ne + e], d1 = pre[(size_t)(3 * nn + 1) * ne + e], d2 = pre[(size_t)(3 * nn + 2) * ne + e];
-#pragma unroll
-    for (int i = 0; i < 3; i++) f[3 * nn + i] = (P[3 * i] * d0 + P[3 * i + 1] * d1 + P[3 * i + 2] * d2) * sixth;
-  }
-#pragma unroll
-  for (int i = 0; i < 3; i++) f[9 + i] = -(f[i] + f[3 + i] + f[6 + i]);
-  if (MODE == 0) {
-#pragma unroll
-    for (int k = 0; k < 12; k++) {
-      int g = gdof[(size_t)k * ne + e];
-      if (g >= 0) fint[g] += f[k];
-    }
-  } else if (MODE == 1) {
-#pragma unroll
-    for (int k = 0; k < 12; k++) out12[(size_t)perm[e] * 12 + k] = f[k];
-  } else {
-#pragma unroll
-    for (int k = 0; k < 12; k++) out12[fst(k, e)] = f[k];
-  }
+  stress_forces<MODE>(U, dvt, Di, vol, out);
+  hyper_stiffness<MODE>(U, VT, Di, T, al, be, vol, sh, out);
 }
 
-template <int MODE, bool DF = false>
-__global__ void __launch_bounds__(128) corot_kernel(int e0, int e1, int ne, const int4* __restrict__ tets,
-                                                    const double* __restrict__ X, const double* __restrict__ u,
-                                                    const double* __restrict__ pre, double thr,
-                                                    const int* __restrict__ emap, const int* __restrict__ gdof,
-                                                    double* __restrict__ K, double* __restrict__ fint,
-                                                    double* __restrict__ out78, double* __restrict__ out12,
-                                                    const int* __restrict__ perm) {
-  const int e = e0 + blockIdx.x * blockDim.x + threadIdx.x;
-  if (e < e1) corot_elem<MODE, DF>(e, ne, tets, X, u, pre, thr, emap, gdof, K, fint, out78, out12, perm);
+template <int MODE>
+__global__ void __launch_bounds__(kElThreads) corot_kernel(int ne, const int4* __restrict__ tets,
+                                                           const double* __restrict__ X, const double* __restrict__ u,
+                                                           const double* __restrict__ pre, double thr, double lambda,
+                                                           double mu, double* __restrict__ out78,
+                                                           double* __restrict__ out12, const int* __restrict__ perm) {
+  __shared__ int2 sa[12][kElThreads];
+  const int e = blockIdx.x * kElThreads + threadIdx.x;
+  if (e < ne) corot_elem<MODE>(e, ne, tets, X, u, pre, thr, lambda, mu, out78, out12, perm, sa);
 }
 
-template <int MODE, bool DF = false>
-__global__ void __launch_bounds__(128) invhyper_kernel(int e0, int e1, int ne, int stvk, const int4* __restrict__ tets,
-                                                       const double* __restrict__ X, const double* __restrict__ u,
-                                                       const double* __restrict__ pre, double thr, double lambda,
-                                                       double mu, const int* __restrict__ emap,
-                                                       const int* __restrict__ gdof, double* __restrict__ K,
-                                                       double* __restrict__ fint, double* __restrict__ out78,
-                                                       double* __restrict__ out12, const int* __restrict__ perm) {
-  const int e = e0 + blockIdx.x * blockDim.x + threadIdx.x;
-  if (e < e1)
-    invhyper_elem<MODE, DF>(e, ne, stvk, tets, X, u, pre, thr, lambda, mu, emap, gdof, K, fint, out78, out12, perm);
+template <int MODE>
+__global__ void __launch_bounds__(kElThreads, kHyperCtas) invhyper_kernel(int ne, int stvk, const int4* __restrict__ tets,
+                                                              const double* __restrict__ X,
+                                                              const double* __restrict__ u,
+                                                              const double* __restrict__ pre, double thr, double lambda,
+                                                              double mu, double* __restrict__ out78,
+                                                              double* __restrict__ out12, const int* __restrict__ perm) {
+  __shared__ HyperShared sh;
+  const int e = blockIdx.x * kElThreads + threadIdx.x;
+  if (e < ne) invhyper_elem<MODE>(e, ne, stvk, tets, X, u, pre, thr, lambda, mu, out78, out12, perm, sh);
 }
 
 // ---- several scenes per launch: tile j of scene s (directory prefix) is
 // its elements [128 j, 128 j + 128); every scene's values land in its own
 // staging arrays
-__global__ void __launch_bounds__(128) corot_batch_kernel(int n_sc, const int* __restrict__ prefix,
-                                                          const SceneDev* __restrict__ sd) {
+__global__ void __launch_bounds__(kElThreads) corot_batch_kernel(int n_sc, const int* __restrict__ prefix,
+                                                                 const SceneDev* __restrict__ sd) {
+  __shared__ int2 sa[12][kElThreads];
   const int s = dir_scene(prefix, n_sc, blockIdx.x);
   const SceneDev& D = sd[s];
-  const int e = (blockIdx.x - prefix[s]) * 128 + threadIdx.x;
+  const int e = (blockIdx.x - prefix[s]) * kElThreads + threadIdx.x;
   if (e >= D.n_tets) return;
-  // batched scenes all run the mixed-precision solver: double-float stiffness
-  corot_elem<2, true>(e, D.n_tets, D.tets, D.X, D.u, D.pre, D.thr, D.emap, D.gdof, nullptr, nullptr, D.stage_k,
-                      D.stage_f, nullptr);
+  corot_elem<2>(e, D.n_tets, D.tets, D.X, D.u, D.pre, D.thr, D.lambda, D.mu, D.stage_k, D.stage_f, nullptr, sa);
 }
 
-__global__ void __launch_bounds__(128) invhyper_batch_kernel(int n_sc, const int* __restrict__ prefix,
-                                                             const SceneDev* __restrict__ sd) {
+__global__ void __launch_bounds__(kElThreads, kHyperCtas) invhyper_batch_kernel(int n_sc, const int* __restrict__ prefix,
+                                                                    const SceneDev* __restrict__ sd) {
+  __shared__ HyperShared sh;
   const int s = dir_scene(prefix, n_sc, blockIdx.x);
   const SceneDev& D = sd[s];
-  const int e = (blockIdx.x - prefix[s]) * 128 + threadIdx.x;
+  const int e = (blockIdx.x - prefix[s]) * kElThreads + threadIdx.x;
   if (e >= D.n_tets) return;
-  // batched scenes all run the mixed-precision solver: double-float contraction
-  invhyper_elem<2, true>(e, D.n_tets, D.kind == OD_MATERIAL_STVK, D.tets, D.X, D.u, D.pre, D.thr, D.lambda, D.mu,
-                         D.emap, D.gdof, nullptr, nullptr, D.stage_k, D.stage_f, nullptr);
+  invhyper_elem<2>(e, D.n_tets, D.kind == OD_MATERIAL_STVK, D.tets, D.X, D.u, D.pre, D.thr, D.lambda, D.mu, D.stage_k,
+                   D.stage_f, nullptr, sh);
 }
 
 // Corotational plastic element (corotationalPlastic.cpp:53-183,
@@ -758,42 +729,18 @@ __global__ void __launch_bounds__(128) invhyper_batch_kernel(int n_sc, const int
 // by creep (|e| - yield)/|e| e and is scaled back to the maximum.  Both
 // norms follow the reference, which adds the squares of the first three
 // entries three times (corotationalPlastic.cpp:156-160, 169-173).
-// pre: [90 K0][9 Dm^-1][V][12 dN] per element (SoA); plastic: [9][ne].
+// plastic: [9][ne].
 template <int MODE>
 __device__ __forceinline__ void plastic_elem(int e, int ne, const int4* __restrict__ tets,
                                              const double* __restrict__ X, const double* __restrict__ u,
                                              const double* __restrict__ pre, double thr, double lambda, double mu,
                                              double yield, double creep, double max_plastic,
                                              double* __restrict__ plastic, double* __restrict__ out78,
-                                             double* __restrict__ out12, const int* __restrict__ perm) {
-  int4 t = tets[e];
-  const int nd[4] = {t.x, t.y, t.z, t.w};
-  V3t<double> c[4];
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    V3t<double> x = ld3(X, nd[i]), du = ld3(u, nd[i]);
-    c[i] = {x.x + du.x, x.y + du.y, x.z + du.z};
-  }
-  double F[9];
-#pragma unroll
-  for (int i = 0; i < 9; i++) F[i] = 0.0;
-#pragma unroll
-  for (int i = 1; i < 4; i++) {
-    double ax[3] = {c[i].x - c[0].x, c[i].y - c[0].y, c[i].z - c[0].z};
-#pragma unroll
-    for (int j = 0; j < 3; j++)
-#pragma unroll
-      for (int k = 0; k < 3; k++) F[j * 3 + k] += ax[j] * pre[(size_t)(90 + (i - 1) * 3 + k) * ne + e];
-  }
-  const double v0 = pre[(size_t)99 * ne + e];
-  const double v1 = tet_vol(c[0], c[1], c[2], c[3]);
-  double R[9], S[9];
-  if (v1 >= thr * v0) polar3<double>(F, R);
-  else qr3<double>(F, R);
-#pragma unroll
-  for (int i = 0; i < 3; i++)
-#pragma unroll
-    for (int j = 0; j < 3; j++) S[i * 3 + j] = R[i] * F[j] + R[3 + i] * F[3 + j] + R[6 + i] * F[6 + j];
+                                             double* __restrict__ out12, const int* __restrict__ perm,
+                                             int2 (*sa)[kElThreads]) {
+  double Di[9], R[9], S[9], v0;
+  corot_frame(e, ne, tets, X, u, pre, thr, Di, v0, R, S);
+  const ElemOut<MODE> out(e, out78, out12, perm);
   // elastic strain, stress, plastic update (computeElasticStress)
   double ep[9], es[9];
 #pragma unroll
@@ -813,11 +760,6 @@ __device__ __forceinline__ void plastic_elem(int e, int ne, const int4* __restri
   st[0] += dg;
   st[4] += dg;
   st[8] += dg;
-  double P[9];
-#pragma unroll
-  for (int i = 0; i < 3; i++)
-#pragma unroll
-    for (int j = 0; j < 3; j++) P[i * 3 + j] = R[i * 3] * st[j] + R[i * 3 + 1] * st[3 + j] + R[i * 3 + 2] * st[6 + j];
   double en = 0.0;  // the reference's sum: each of the first three squares three times, in its order
 #pragma unroll
   for (int i = 0; i < 3; i++) {
@@ -846,82 +788,33 @@ __device__ __forceinline__ void plastic_elem(int e, int ne, const int4* __restri
 #pragma unroll
     for (int i = 0; i < 9; i++) plastic[(size_t)i * ne + e] = ep[i];
   }
-  auto put = [&](int k, double val) {
-    if (MODE == 1) out78[(size_t)perm[e] * 78 + k] = val;
-    else out78[kst(k, e)] = val;
-  };
-  int blk = 0;
-#pragma unroll 1
-  for (int a = 0; a < 4; a++) {
-#pragma unroll 1
-    for (int b = a; b < 4; b++) {
-      double K0[9], QK[9], QKQT[9];
-#pragma unroll
-      for (int i = 0; i < 9; i++) K0[i] = pre[(size_t)(9 * blk + i) * ne + e];
-      blk++;
-#pragma unroll
-      for (int i = 0; i < 3; i++)
-#pragma unroll
-        for (int j = 0; j < 3; j++) QK[i * 3 + j] = R[i * 3] * K0[j] + R[i * 3 + 1] * K0[3 + j] + R[i * 3 + 2] * K0[6 + j];
-#pragma unroll
-      for (int i = 0; i < 3; i++)
-#pragma unroll
-        for (int j = 0; j < 3; j++)
-          QKQT[i * 3 + j] = QK[i * 3] * R[j * 3] + QK[i * 3 + 1] * R[j * 3 + 1] + QK[i * 3 + 2] * R[j * 3 + 2];
-      if (a == b) {
-#pragma unroll
-        for (int i = 0; i < 3; i++)
-#pragma unroll
-          for (int j = 0; j < 3 - i; j++) put(c_diag12[a * 3 + i] + j, QKQT[i * 3 + i + j]);
-      } else {
-#pragma unroll
-        for (int i = 0; i < 3; i++)
-#pragma unroll
-          for (int j = 0; j < 3; j++) put(c_diag12[a * 3 + i] + (b - a) * 3 - i + j, QKQT[i * 3 + j]);
-      }
-    }
-  }
-  double f[12];
-  const double sixth = 1.0 / 6.0;
-#pragma unroll
-  for (int n = 0; n < 3; n++) {
-    const double x = pre[(size_t)(100 + 3 * n) * ne + e], y = pre[(size_t)(101 + 3 * n) * ne + e],
-                 z = pre[(size_t)(102 + 3 * n) * ne + e];
-#pragma unroll
-    for (int i = 0; i < 3; i++) f[3 * n + i] = (P[i * 3] * x + P[i * 3 + 1] * y + P[i * 3 + 2] * z) * sixth;
-  }
-#pragma unroll
-  for (int i = 0; i < 3; i++) f[9 + i] = -(f[i] + f[3 + i] + f[6 + i]);
-  if (MODE == 1) {
-#pragma unroll
-    for (int k = 0; k < 12; k++) out12[(size_t)perm[e] * 12 + k] = f[k];
-  } else {
-#pragma unroll
-    for (int k = 0; k < 12; k++) out12[fst(k, e)] = f[k];
-  }
+  stress_forces<MODE>(R, st, Di, v0, out);
+  corot_stiffness<MODE>(R, Di, lambda * v0, mu * v0, sa, out);
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(128) plastic_kernel(int ne, const int4* __restrict__ tets,
+__global__ void __launch_bounds__(kElThreads) plastic_kernel(int ne, const int4* __restrict__ tets,
                                                       const double* __restrict__ X, const double* __restrict__ u,
                                                       const double* __restrict__ pre, double thr, double lambda,
                                                       double mu, double yield, double creep, double max_plastic,
                                                       double* __restrict__ plastic, double* __restrict__ out78,
                                                       double* __restrict__ out12, const int* __restrict__ perm) {
+  __shared__ int2 sa[12][kElThreads];
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e < ne)
     plastic_elem<MODE>(e, ne, tets, X, u, pre, thr, lambda, mu, yield, creep, max_plastic, plastic, out78, out12,
-                       perm);
+                       perm, sa);
 }
 
-__global__ void __launch_bounds__(128) plastic_batch_kernel(int n_sc, const int* __restrict__ prefix,
-                                                            const SceneDev* __restrict__ sd) {
+__global__ void __launch_bounds__(kElThreads) plastic_batch_kernel(int n_sc, const int* __restrict__ prefix,
+                                                                   const SceneDev* __restrict__ sd) {
+  __shared__ int2 sa[12][kElThreads];
   const int s = dir_scene(prefix, n_sc, blockIdx.x);
   const SceneDev& D = sd[s];
   const int e = (blockIdx.x - prefix[s]) * 128 + threadIdx.x;
   if (e >= D.n_tets) return;
   plastic_elem<2>(e, D.n_tets, D.tets, D.X, D.u, D.pre, D.thr, D.lambda, D.mu, D.yield, D.creep, D.max_plastic,
-                  D.plastic, D.stage_k, D.stage_f, nullptr);
+                  D.plastic, D.stage_k, D.stage_f, nullptr, sa);
 }
 
 // atomic-free scatter of staged element values, one colour per launch
@@ -1168,8 +1061,7 @@ od_status launch_precompute(Scene* s) {
   const int T = 128;
   if (s->n_tets == 0) return OD_OK;
   OD_KL(s);
-  precompute_kernel<<<nblk(s->n_tets, T), T, 0, s->ctx->stream>>>(s->n_tets, s->mat.kind, s->tets, s->X, s->D[0],
-                                                                   s->D[1], s->D[2], s->pre);
+  precompute_kernel<<<nblk(s->n_tets, T), T, 0, s->ctx->stream>>>(s->n_tets, s->tets, s->X, s->pre);
   OD_CUDA(cudaGetLastError());
   return OD_OK;
 }
@@ -1256,10 +1148,6 @@ od_status launch_hooke(Scene* s, double youngs, double poisson, double* Kh) {
   return OD_OK;
 }
 
-static int vol_slot(const Scene* s) {
-  return s->mat.kind == OD_MATERIAL_COROTATIONAL || s->mat.kind == OD_MATERIAL_COROTATIONAL_PLASTIC ? 99 : 21;
-}
-
 od_status launch_mass(Scene* s) {
   const int T = 128;
   OD_CUDA(cudaMemsetAsync(s->M, 0, sizeof(double) * (size_t)s->nvals, s->ctx->stream));
@@ -1268,18 +1156,18 @@ od_status launch_mass(Scene* s) {
     int e0 = s->color_off[c], e1 = s->color_off[c + 1];
     if (e1 <= e0) continue;
     OD_KL(s);
-    mass_kernel<<<nblk(e1 - e0, T), T, 0, s->ctx->stream>>>(e0, e1, s->n_tets, vol_slot(s), s->mat.density, s->pre,
+    mass_kernel<<<nblk(e1 - e0, T), T, 0, s->ctx->stream>>>(e0, e1, s->n_tets, s->mat.density, s->pre,
                                                              s->emap, s->M);
     OD_KL(s);
-    node_vol_kernel<<<nblk(e1 - e0, T), T, 0, s->ctx->stream>>>(e0, e1, s->n_tets, vol_slot(s), s->tets, s->pre,
+    node_vol_kernel<<<nblk(e1 - e0, T), T, 0, s->ctx->stream>>>(e0, e1, s->n_tets, s->tets, s->pre,
                                                                  s->node_vol4);
   }
   OD_CUDA(cudaGetLastError());
   return OD_OK;
 }
 
-od_status launch_eval(Scene* s, bool zero_first, bool df) {
-  const int T = 128;
+od_status launch_eval(Scene* s, bool zero_first) {
+  const int T = kElThreads;
   cudaStream_t st = s->ctx->stream;
   if (zero_first && (!s->gat_kptr || s->n_tets == 0)) {
     OD_CUDA(cudaMemsetAsync(s->K, 0, sizeof(double) * (size_t)s->nvals, st));
@@ -1293,24 +1181,12 @@ od_status launch_eval(Scene* s, bool zero_first, bool df) {
                                                          s->lambda, s->mu, s->mat.yield_criterion,
                                                          s->mat.creep_ratio, s->mat.max_plastic_strain, s->plastic,
                                                          s->stage_k, s->stage_f, nullptr);
-  else if (s->mat.kind == OD_MATERIAL_COROTATIONAL && df)
-    corot_kernel<2, true><<<nblk(s->n_tets, T), T, 0, st>>>(0, s->n_tets, s->n_tets, s->tets, s->X, s->u, s->pre,
-                                                             s->mat.threshold, s->emap, s->gdof, nullptr, nullptr,
-                                                             s->stage_k, s->stage_f, nullptr);
   else if (s->mat.kind == OD_MATERIAL_COROTATIONAL)
-    corot_kernel<2><<<nblk(s->n_tets, T), T, 0, st>>>(0, s->n_tets, s->n_tets, s->tets, s->X, s->u, s->pre,
-                                                       s->mat.threshold, s->emap, s->gdof, nullptr, nullptr, s->stage_k,
-                                                       s->stage_f, nullptr);
-  else if (df)
-    invhyper_kernel<2, true><<<nblk(s->n_tets, T), T, 0, st>>>(0, s->n_tets, s->n_tets,
-                                                                s->mat.kind == OD_MATERIAL_STVK, s->tets, s->X, s->u,
-                                                                s->pre, s->mat.threshold, s->lambda, s->mu, s->emap,
-                                                                s->gdof, nullptr, nullptr, s->stage_k, s->stage_f,
-                                                                nullptr);
+    corot_kernel<2><<<nblk(s->n_tets, T), T, 0, st>>>(s->n_tets, s->tets, s->X, s->u, s->pre, s->mat.threshold,
+                                                      s->lambda, s->mu, s->stage_k, s->stage_f, nullptr);
   else
-    invhyper_kernel<2><<<nblk(s->n_tets, T), T, 0, st>>>(0, s->n_tets, s->n_tets, s->mat.kind == OD_MATERIAL_STVK,
-                                                          s->tets, s->X, s->u, s->pre, s->mat.threshold, s->lambda,
-                                                          s->mu, s->emap, s->gdof, nullptr, nullptr, s->stage_k,
+    invhyper_kernel<2><<<nblk(s->n_tets, T), T, 0, st>>>(s->n_tets, s->mat.kind == OD_MATERIAL_STVK, s->tets, s->X, s->u,
+                                                          s->pre, s->mat.threshold, s->lambda, s->mu, s->stage_k,
                                                           s->stage_f, nullptr);
   // 2) assembly: one gather launch; one scatter launch per colour for meshes
   //    whose gather lists do not fit 32-bit indices
@@ -1335,7 +1211,7 @@ od_status launch_eval(Scene* s, bool zero_first, bool df) {
 }
 
 od_status launch_element_values(Scene* s, double* d_k78, double* d_f12) {
-  const int T = 128;
+  const int T = kElThreads;
   cudaStream_t st = s->ctx->stream;
   if (s->n_tets == 0) return OD_OK;
   OD_KL(s);
@@ -1345,13 +1221,11 @@ od_status launch_element_values(Scene* s, double* d_k78, double* d_f12) {
                                                          s->mat.creep_ratio, s->mat.max_plastic_strain, s->plastic,
                                                          d_k78, d_f12, s->perm);
   else if (s->mat.kind == OD_MATERIAL_COROTATIONAL)
-    corot_kernel<1><<<nblk(s->n_tets, T), T, 0, st>>>(0, s->n_tets, s->n_tets, s->tets, s->X, s->u, s->pre,
-                                                       s->mat.threshold, s->emap, s->gdof, nullptr, nullptr, d_k78,
-                                                       d_f12, s->perm);
+    corot_kernel<1><<<nblk(s->n_tets, T), T, 0, st>>>(s->n_tets, s->tets, s->X, s->u, s->pre, s->mat.threshold,
+                                                      s->lambda, s->mu, d_k78, d_f12, s->perm);
   else
-    invhyper_kernel<1><<<nblk(s->n_tets, T), T, 0, st>>>(0, s->n_tets, s->n_tets, s->mat.kind == OD_MATERIAL_STVK,
-                                                          s->tets, s->X, s->u, s->pre, s->mat.threshold, s->lambda,
-                                                          s->mu, s->emap, s->gdof, nullptr, nullptr, d_k78, d_f12,
+    invhyper_kernel<1><<<nblk(s->n_tets, T), T, 0, st>>>(s->n_tets, s->mat.kind == OD_MATERIAL_STVK, s->tets, s->X, s->u,
+                                                          s->pre, s->mat.threshold, s->lambda, s->mu, d_k78, d_f12,
                                                           s->perm);
   OD_CUDA(cudaGetLastError());
   return OD_OK;

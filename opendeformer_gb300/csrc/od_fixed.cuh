@@ -82,6 +82,20 @@ struct FxAcc {
   }
 };
 
+// A sum of products of operands at scales Ea and Eb as digits at the scale
+// Ea + Eb + (sh - 2); sh >= 1.
+__device__ __forceinline__ int2 fx_split(long long x) {
+  const int h = (int)((x + (1LL << (kFxLow - 1))) >> kFxLow);
+  return make_int2(h, (int)((unsigned)x - ((unsigned)h << kFxLow)));
+}
+__device__ __forceinline__ int2 fx_norm(const FxAcc& c, int sh) {
+  return fx_split((c.hh + (c.mid >> kFxLow) + (1LL << (sh - 1))) >> sh);
+}
+// The same sum as FP64, to 2^-62 of its scale 2^E, E = Ea + Eb.
+__device__ __forceinline__ double fx_out(const FxAcc& c, int E) {
+  return fx_double(c.hh + (c.mid >> kFxLow), E - 2 * (kFxBits - kFxLow));
+}
+
 // An FP64 addition holds a warp's unit for 64 cycles, so sums across a warp
 // are integer sums too: every addend aligned to the largest exponent em
 // (a multiple of 2^(em - 1075 - up)), added as 64-bit integers.  A warp-wide

@@ -4,8 +4,7 @@
 // colour order so every colour is a contiguous range):
 //   X, u            n_nodes*3 double   rest positions / mesh displacement
 //   tets            n_tets int4        node ids
-//   pre             SoA [k][n_tets]    corotational: 90 K0 + 9 Dm^-1 + V;
-//                                      invertible:   12 dN + 9 Dm^-1 + V
+//   pre             SoA [k][n_tets]    9 Dm^-1 + V
 //   emap            SoA [78][n_tets]   reference element->value map
 //   gdof            SoA [12][n_tets]   compacted DOF of each element DOF or -1
 //   K, M, D         n_values double    tangent / mass / external damping in the
@@ -504,7 +503,8 @@ od_status launch_precompute(Scene* s);
 od_status launch_mass(Scene* s);
 // K, fint at current u; df: the mixed-precision path's double-float stiffness
 // contraction (invertible materials; the others are unchanged)
-od_status launch_eval(Scene* s, bool zero_first, bool df = false);
+od_status launch_eval(Scene* s, bool zero_first);
+int element_precomputes();   // doubles per element in Scene::pre
 od_status launch_hooke(Scene* s, double youngs, double poisson, double* Kh);  // linear K, reference layout
 // new body force / uniform traction on the facets of the last od_scene_set_loads
 od_status scene_set_uniform_loads(Scene* s, const double* body, const double* traction);

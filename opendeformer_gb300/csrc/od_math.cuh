@@ -51,6 +51,17 @@ template <class FT> __device__ __forceinline__ void mul3(const FT* a, const FT* 
     for (int j = 0; j < 3; j++) c[3 * i + j] = a[3 * i] * b[j] + a[3 * i + 1] * b[3 + j] + a[3 * i + 2] * b[6 + j];
 }
 
+// x to float by its bits, cut to 24 bits (the FP64 units also run FP64 <->
+// FP32 conversions); 0 below the normal range, infinity (or NaN) above it
+__device__ __forceinline__ float cut_float(double x) {
+  const int hi = __double2hiint(x), e = (hi >> 20) & 0x7ff;
+  const unsigned m = ((unsigned)hi << 3) | ((unsigned)__double2loint(x) >> 29);
+  unsigned u = ((unsigned)(e - 896) << 23) | (m & 0x7fffffu);
+  if (e <= 896) u = 0;
+  if (e >= 1151) u = 0x7f800000u | (e == 0x7ff ? m & 0x7fffffu : 0u);
+  return __uint_as_float(u | ((unsigned)hi & 0x80000000u));
+}
+
 // Symmetric 3x3 eigen-decomposition, eigenvectors as rows
 // (eigenSym3x3, core/numerMethod.h:327-429): trigonometric root for the
 // first eigenvalue, then a 2x2 problem on its orthogonal complement.
@@ -58,8 +69,10 @@ template <class FT> __device__ __forceinline__ void mul3(const FT* a, const FT* 
 // steps on the deviator's characteristic polynomial l^3 - J2 l - J3 (the
 // chosen root is the one of largest magnitude, where the derivative
 // 3 l^2 - J2 is at least 2 J2, so the FP32 start's ~1e-7 error falls below
-// FP64 rounding); FP64 transcendental functions are long instruction
-// sequences on the FP64 pipe.
+// FP64 rounding, and the derivative's reciprocal need not be better than
+// FP32 either); FP64 roots, quotients and transcendental functions are long
+// instruction sequences on the FP64 pipe.  Deviators whose J2 FP32 cannot
+// hold well take the FP64 expressions.
 template <class FT, bool REFINE = false>
 __device__ void eig_sym3(const FT* t, FT* vals, FT* vecs) {
   const FT pi = FT(3.141592653589793238462643383279502884);
@@ -70,26 +83,33 @@ __device__ void eig_sym3(const FT* t, FT* vals, FT* vecs) {
   const FT d0 = t[0] - ave, d1 = t[3] - ave, d2 = t[5] - ave;
   const FT J2 = (d0 * d0 + d1 * d1 + d2 * d2) * FT(0.5) + t[1] * t[1] + t[2] * t[2] + t[4] * t[4];
   const FT J3 = d0 * (d1 * d2 - t[4] * t[4]) + t[1] * (t[4] * t[2] - t[1] * d2) + t[2] * (t[1] * t[4] - d1 * t[2]);
-  const FT sq = sqrt(J2);
-  const FT cs = REFINE ? (FT(3) * FT(0.5) * s3) * (J3 / (J2 * sq)) : (FT(3) * FT(0.5) * s3) * ((J3 / J2) / sq);
-  if (isnan(cs) || isinf(cs)) {
-    vals[0] = vals[1] = vals[2] = ave;
-#pragma unroll
-    for (int i = 0; i < 9; i++) vecs[i] = FT(0);
-    vecs[0] = vecs[4] = vecs[8] = FT(1);
-    return;
-  }
   FT e0;
+  bool started = false;
   if constexpr (REFINE) {
-    const float pif = 3.14159265358979f;
-    const float angf = acosf((float)clampv(cs, FT(-1), FT(1))) / 3.f;
-    const float cf = angf < pif / 6.f ? cosf(angf) : cosf(angf + (2.f / 3.f) * pif);
-    e0 = (FT(2) / s3) * sq * (FT)cf;
-    const FT rdp = FT(1) / (FT(3) * e0 * e0 - J2);
-    e0 -= ((e0 * e0 - J2) * e0 - J3) * rdp;
-    e0 -= ((e0 * e0 - J2) * e0 - J3) * rdp;
-  } else {
-    FT ang = acos(clampv(cs, FT(-1), FT(1))) / FT(3);
+    const float j2 = cut_float(J2);
+    if (j2 > 1e-24f && j2 < 1e20f) {
+      const float pif = 3.14159265358979f, ri = rsqrtf(j2);
+      const float cs = 2.59807621f * cut_float(J3) * ri * ri * ri;
+      const float ang = acosf(fminf(fmaxf(cs, -1.f), 1.f)) / 3.f;
+      const float ef = 1.15470054f * (j2 * ri) * (ang < pif / 6.f ? cosf(ang) : cosf(ang + (2.f / 3.f) * pif));
+      const FT rdp = (FT)(1.f / (3.f * ef * ef - j2));
+      e0 = (FT)ef;
+      e0 -= ((e0 * e0 - J2) * e0 - J3) * rdp;
+      e0 -= ((e0 * e0 - J2) * e0 - J3) * rdp;
+      started = true;
+    }
+  }
+  if (!started) {
+    const FT sq = sqrt(J2);
+    const FT cs = (FT(3) * FT(0.5) * s3) * ((J3 / J2) / sq);
+    if (isnan(cs) || isinf(cs)) {
+      vals[0] = vals[1] = vals[2] = ave;
+#pragma unroll
+      for (int i = 0; i < 9; i++) vecs[i] = FT(0);
+      vecs[0] = vecs[4] = vecs[8] = FT(1);
+      return;
+    }
+    const FT ang = acos(clampv(cs, FT(-1), FT(1))) / FT(3);
     e0 = (FT(2) / s3) * sq * (ang < pi / FT(6) ? cos(ang) : cos(ang + (FT(2) / FT(3)) * pi));
   }
   vals[0] = e0 + ave;
@@ -248,8 +268,9 @@ __device__ void polar3(const FT* F, FT* R) {
     R[0] = R[4] = R[8] = FT(1);
     return;
   }
+  const FT rfn = FT(1) / fn;
 #pragma unroll
-  for (int i = 0; i < 9; i++) A[i] = F[i] / fn;
+  for (int i = 0; i < 9; i++) A[i] = F[i] * rfn;
   FT b = FT(0), t;
   t = A[4] * A[8] - A[5] * A[7]; b += t * t;
   t = A[3] * A[8] - A[5] * A[6]; b += t * t;
@@ -270,30 +291,7 @@ __device__ void polar3(const FT* F, FT* R) {
   const FT tau = FT(1e-4);
   const bool quick = b <= FT(1) - tau;
   if (quick) {
-    int perm0 = 1, perm1 = 2;
-    int rowIndex = 0;
-    FT largest = fabs(A[0]);
-    if (fabs(A[3]) > largest) { largest = fabs(A[3]); rowIndex = 1; }
-    if (fabs(A[6]) > largest) rowIndex = 2;
-    if (rowIndex != 0) { dA = -dA; if (rowIndex == 1) perm0 = 0; else perm1 = 0; }
-    const int row = rowIndex;
-    FT piv = A[row * 3];
-    dA *= piv;
-    if (dA != FT(0)) {
-      FT lo = A[perm0 * 3] / piv;
-      A[perm0 * 3 + 1] -= lo * A[row * 3 + 1];
-      A[perm0 * 3 + 2] -= lo * A[row * 3 + 2];
-      lo = A[perm1 * 3] / piv;
-      A[perm1 * 3 + 1] -= lo * A[row * 3 + 1];
-      A[perm1 * 3 + 2] -= lo * A[row * 3 + 2];
-      int r2, s2;
-      if (fabs(A[perm0 * 3 + 1]) > fabs(A[perm1 * 3 + 1])) { r2 = perm0; s2 = perm1; }
-      else { dA = -dA; r2 = perm1; s2 = perm0; }
-      FT p2 = A[r2 * 3 + 1];
-      dA *= p2;
-      FT lo2 = A[s2 * 3 + 1] / p2;
-      dA *= (A[s2 * 3 + 2] - lo2 * A[r2 * 3 + 2]);
-    }
+    dA = det3(A);
   } else {
     int rp[3] = {0, 1, 2}, cp[3] = {0, 1, 2};
     for (int i = 0; i < 2; i++) {
@@ -328,15 +326,30 @@ __device__ void polar3(const FT* F, FT* R) {
   const FT inv3 = FT(0.333333333333333333333333);
   FT lam;
   if (b >= tau - inv3) {
-    FT c = FT(8) * dA;
-    FT D0 = FT(1) + FT(3) * b;
-    FT D1 = FT(-1) + (FT(27) / FT(16)) * c * c + FT(9) * b;
-    FT sD0 = sqrt(D0);
-    FT al = D1 / (D0 * sD0);
-    FT z = (FT(4) * inv3) * (FT(1) + sD0 * cos(acos(clampv(al, FT(-1), FT(1))) * inv3));
-    FT s = sqrt(z) * FT(0.5);
-    FT arg = FT(4) - z + c / s;
-    lam = s + FT(0.5) * sqrt(arg > FT(0) ? arg : FT(0));
+    // the closed form in FP32, then two Newton steps (the derivative's
+    // reciprocal need not be better than FP32) -- FP64 roots, quotients and
+    // transcendental functions are long sequences on the FP64 units; the
+    // closed form in FP64 where the root is close to another
+    const FT c = FT(8) * dA;
+    const float cf = (float)c, bf = (float)b;
+    const float d0 = 1.f + 3.f * bf, s0 = sqrtf(d0), al0 = (-1.f + (27.f / 16.f) * cf * cf + 9.f * bf) / (d0 * s0);
+    const float z0 = (4.f / 3.f) * (1.f + s0 * cosf(acosf(fminf(fmaxf(al0, -1.f), 1.f)) / 3.f)), r0 = sqrtf(z0) * 0.5f;
+    const float l0 = r0 + 0.5f * sqrtf(fmaxf(4.f - z0 + cf / r0, 0.f)), df = 4.f * l0 * (l0 * l0 - 1.f) - cf;
+    if (df > 0.05f) {
+      const FT rd = (FT)(1.f / df);
+      lam = (FT)l0;
+      lam -= (lam * (lam * (lam * lam - FT(2)) - c) + b) * rd;
+      lam -= (lam * (lam * (lam * lam - FT(2)) - c) + b) * rd;
+    } else {
+      FT D0 = FT(1) + FT(3) * b;
+      FT D1 = FT(-1) + (FT(27) / FT(16)) * c * c + FT(9) * b;
+      FT sD0 = sqrt(D0);
+      FT al = D1 / (D0 * sD0);
+      FT z = (FT(4) * inv3) * (FT(1) + sD0 * cos(acos(clampv(al, FT(-1), FT(1))) * inv3));
+      FT s = sqrt(z) * FT(0.5);
+      FT arg = FT(4) - z + c / s;
+      lam = s + FT(0.5) * sqrt(arg > FT(0) ? arg : FT(0));
+    }
   } else {
     lam = FT(1.7320508075688772935274463415058723669428);
     FT old;
@@ -362,9 +375,10 @@ __device__ void polar3(const FT* F, FT* R) {
     }
     if (di != 0) { int tt = ix[0]; ix[0] = ix[di]; ix[di] = tt; }
     int p = ix[0];
-    L[0] = B[p * 4 + ix[1]] / largest;
-    L[1] = B[p * 4 + ix[2]] / largest;
-    L[2] = B[p * 4 + ix[3]] / largest;
+    const FT rl = FT(1) / largest;
+    L[0] = B[p * 4 + ix[1]] * rl;
+    L[1] = B[p * 4 + ix[2]] * rl;
+    L[2] = B[p * 4 + ix[3]] * rl;
     int r = ix[1], c;
     FT od;
     B[r * 5] -= L[0] * B[p * 4 + r];
@@ -388,8 +402,9 @@ __device__ void polar3(const FT* F, FT* R) {
       FT tl = L[0]; L[0] = L[di - 1]; L[di - 1] = tl;
     }
     p = ix[1];
-    L[3] = B[p * 4 + ix[2]] / largest;
-    L[4] = B[p * 4 + ix[3]] / largest;
+    const FT rl = FT(1) / largest;
+    L[3] = B[p * 4 + ix[2]] * rl;
+    L[4] = B[p * 4 + ix[3]] * rl;
     int r = ix[2], c = ix[3];
     B[r * 5] -= L[3] * B[p * 4 + r];
     FT od = B[r * 4 + c] - L[3] * B[p * 4 + c];
@@ -505,9 +520,9 @@ __device__ void polar3(const FT* F, FT* R) {
       }
     }
   }
-  FT nn = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2] + v[3] * v[3]);
+  const FT rn = FT(1) / sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2] + v[3] * v[3]);
 #pragma unroll
-  for (int i = 0; i < 4; i++) v[i] /= nn;
+  for (int i = 0; i < 4; i++) v[i] *= rn;
   const FT v11 = v[1] * v[1], v22 = v[2] * v[2], v33 = v[3] * v[3];
   const FT v12 = v[1] * v[2], v03 = v[0] * v[3], v13 = v[1] * v[3];
   const FT v02 = v[0] * v[2], v23 = v[2] * v[3], v01 = v[0] * v[1];
@@ -544,8 +559,7 @@ __device__ void invertible_svd(const FT* F, FT thr, FT* sig, FT* U, FT* VT) {
   tri[3] = F[3] * F[3] + F[4] * F[4] + F[5] * F[5];
   tri[4] = F[6] * F[3] + F[7] * F[4] + F[8] * F[5];
   tri[5] = F[6] * F[6] + F[7] * F[7] + F[8] * F[8];
-  eig_sym3<FT, REFINE>(tri, ev, UT);
-  if (det3(UT) < FT(0)) { UT[0] = -UT[0]; UT[1] = -UT[1]; UT[2] = -UT[2]; }
+  eig_sym3<FT, REFINE>(tri, ev, UT);   // rows e0, e1, e0 x e1: a rotation
   // REFINE: sigma = x rsqrt(x), and rsqrt(x) is 1 / sigma for the row scaling
   FT rs[3];
 #pragma unroll
@@ -567,7 +581,11 @@ __device__ void invertible_svd(const FT* F, FT thr, FT* sig, FT* U, FT* VT) {
   switch (cond) {
     case 0: {
       scalerow(0, inv(0)); scalerow(1, inv(1)); scalerow(2, inv(2));
-      if (det3(VT) < FT(0)) {
+      // orthonormal rows: det V is 1 or -1 up to rounding
+      float vt[9];
+#pragma unroll
+      for (int i = 0; i < 9; i++) vt[i] = cut_float(VT[i]);
+      if (det3(vt) < 0.f) {
         int sm = ev[0] < ev[1] ? (ev[0] < ev[2] ? 0 : 2) : (ev[1] < ev[2] ? 1 : 2);
         scalerow(sm, FT(-1));
         ev[sm] = -ev[sm];
@@ -599,6 +617,17 @@ template <class FT>
 __device__ void psd3(FT* m) {
   // Positive leading minors (Sylvester) prove every eigenvalue positive, in
   // which case the projection leaves the matrix unchanged: skip the eigensolve.
+  // (in FP32 first: minors far enough above their rounding settle it)
+  {
+    float f[6];
+#pragma unroll
+    for (int i = 0; i < 6; i++) f[i] = cut_float(m[i]);
+    const float c0 = f[3] * f[5] - f[4] * f[4], c1 = f[1] * f[5] - f[4] * f[2], c2 = f[1] * f[4] - f[3] * f[2];
+    const float m01 = f[0] * f[3] - f[1] * f[1], dt = f[0] * c0 - f[1] * c1 + f[2] * c2;
+    const float big = fabsf(f[0]) * (fabsf(f[3] * f[5]) + f[4] * f[4]) + fabsf(f[1]) * (fabsf(f[1] * f[5]) + fabsf(f[4] * f[2])) +
+                      fabsf(f[2]) * (fabsf(f[1] * f[4]) + fabsf(f[3] * f[2]));
+    if (f[0] > 0.f && m01 > 1e-5f * fabsf(f[0] * f[3]) && dt > 1e-5f * big && big < 1e37f) return;
+  }
   {
     const FT m01 = m[0] * m[3] - m[1] * m[1];
     const FT dt = m[0] * (m[3] * m[5] - m[4] * m[4]) - m[1] * (m[1] * m[5] - m[4] * m[2]) +
@@ -606,7 +635,7 @@ __device__ void psd3(FT* m) {
     if (m[0] > FT(0) && m01 > FT(0) && dt > FT(0)) return;
   }
   FT QT[9], ev[3];
-  eig_sym3(m, ev, QT);
+  eig_sym3<FT, true>(m, ev, QT);
   bool neg = false;
 #pragma unroll
   for (int i = 0; i < 3; i++) if (ev[i] < FT(0)) { neg = true; ev[i] = FT(0); }
