@@ -501,8 +501,7 @@ void ric_factor(const RicColumns& A, const double* values, double eps, double re
 // ---- kernels (od_elements.cu) ----
 od_status launch_precompute(Scene* s);
 od_status launch_mass(Scene* s);
-// K, fint at current u; df: the mixed-precision path's double-float stiffness
-// contraction (invertible materials; the others are unchanged)
+// K, fint at current u
 od_status launch_eval(Scene* s, bool zero_first);
 int element_precomputes();   // doubles per element in Scene::pre
 od_status launch_hooke(Scene* s, double youngs, double poisson, double* Kh);  // linear K, reference layout
