@@ -145,6 +145,8 @@ struct Pcg {
   // solve (both built on first use)
   SliceSys* slice = nullptr;
   MixedSys* mix = nullptr;
+  bool icp_tried = false;
+  struct IcPcg* icp = nullptr;  // the one-launch IC(0) PCG's structure (od_ic_pcg.cu); null: not taken
   struct MixIc0* mic = nullptr;  // mixed precision with IC(0) (FP32 factor copy and inner vectors)
   // incomplete LDL^T / threshold incomplete Cholesky (factor on the host,
   // triangular sweeps on the device)
@@ -611,6 +613,11 @@ od_status resident_plan(Scene* s);
 void resident_free(ResidentPlan* R);
 od_status resident_solve(Scene* s, const double* d_b, double* d_x, int pkind, double tol, int max_iter, bool x_zero,
                          unsigned long long* prof);
+// the one-launch PCG with IC(0) in colour order (od_ic_pcg.cu)
+od_status ic_pcg_build(Scene* s, const std::vector<int>& rp, const std::vector<int>& col, const std::vector<int>& order,
+                       const std::vector<int>& cstart, IcPcg** out);
+od_status ic_pcg_solve(Scene* s, IcPcg* I, const double* d_b, double* d_x, double tol, int max_iter);
+void ic_pcg_free(IcPcg* I);
 od_status pcg_solve(Scene* s, const double* d_b, double* d_x, const od_solver_params* prm, od_solve_stats* st);
 
 // ---- mixed-precision systems (od_sparse.cu)

@@ -2482,6 +2482,25 @@ static od_status ic0_build(Scene* s) {
   return OD_OK;
 }
 
+// The one-launch PCG's structure, built at the first solve that may use it:
+// blocks in colour order and none of the switches that ask for the separate
+// launches.  P.icp stays null where it does not take the system.
+static od_status ic0_one_launch(Scene* s) {
+  Pcg& P = s->pcg;
+  if (P.icp_tried) return OD_OK;
+  P.icp_tried = true;
+  const char* order = std::getenv("OD_GB300_IC0_ORDER");
+  if (std::getenv("OD_GB300_IC0_FACTOR") || std::getenv("OD_GB300_IC0_SWEEP") ||
+      (order && std::strcmp(order, "natural") == 0))
+    return OD_OK;
+  const int nb = s->bsr.nb;
+  std::vector<int> rp(nb + 1), col(s->bsr.nnzb), perm(nb), cstart;
+  OD_CUDA(cudaMemcpy(rp.data(), s->bsr.row_ptr, sizeof(int) * (nb + 1), cudaMemcpyDeviceToHost));
+  OD_CUDA(cudaMemcpy(col.data(), s->bsr.col, sizeof(int) * s->bsr.nnzb, cudaMemcpyDeviceToHost));
+  ic0_colour_order(nb, rp, col, perm, cstart);
+  return ic_pcg_build(s, rp, col, perm, cstart, &P.icp);
+}
+
 od_status ic0_check(Scene* s);
 
 // shifted IC(0) factorisation of the current A64 with the Manteuffel retry
@@ -2681,6 +2700,7 @@ void pcg_free(Scene* s) {
   cudaFree(P.gbar);
   mixed_free(P.mix);
   mixed_ic0_free(P.mic);
+  ic_pcg_free(P.icp);
   slice_free(P.slice);
   sweep_free(P.sweep);
   resident_free(&P.res);
@@ -3333,6 +3353,16 @@ od_status pcg_solve(Scene* s, const double* d_b, double* d_x, const od_solver_pa
     OD_KL(s);
     precond_setup_kernel<double><<<nblk(nb, kThreads), kThreads, 0, strm>>>(nb, pk, s->bsr.diag_pos, s->A64, P.pinv);
   } else if (pk == OD_PRECOND_IC0) {
+    OD_TRY(ic0_one_launch(s));
+    if (P.icp) {
+      const bool prof = s->ctx->profiling && s->ctx->ev_pool.size() >= 2;
+      if (prof) OD_CUDA(cudaEventRecord(s->ctx->ev_pool[0], strm));
+      OD_TRY(ic_pcg_solve(s, P.icp, d_b, d_x, prm->tol, prm->max_iter));
+      if (prof) OD_CUDA(cudaEventRecord(s->ctx->ev_pool[1], strm));
+      od_status e = pcg_finish(s, d_b, d_x, 0.0, st, true, prof);
+      if (st) st->ic_shift = P.sc_host->alpha;
+      return e;
+    }
     od_status e = ic0_factor(s);
     if (e != OD_OK) return e;
     shift = P.ic_shift;
