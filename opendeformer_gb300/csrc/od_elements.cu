@@ -600,7 +600,7 @@ __device__ __forceinline__ void invhyper_elem(int e, int ne, int stvk, const int
                                               const double* __restrict__ X, const double* __restrict__ u,
                                               const double* __restrict__ pre, double thr, double lambda, double mu,
                                               double* __restrict__ out78, double* __restrict__ out12,
-                                              const int* __restrict__ perm, HyperShared& sh) {
+                                              const int* __restrict__ perm, bool refine, HyperShared& sh) {
   int4 t = tets[e];
   const int nd[4] = {t.x, t.y, t.z, t.w};
   V3t<double> c[4];
@@ -621,7 +621,10 @@ __device__ __forceinline__ void invhyper_elem(int e, int ne, int stvk, const int
       for (int k = 0; k < 3; k++) F[j * 3 + k] += ax[j] * Di[(i - 1) * 3 + k];
   }
   double sig[3], U[9], VT[9];
-  invertible_svd<double, true>(F, thr, sig, U, VT);
+  if (!invertible_svd<double, true, false>(F, thr, sig, U, VT)) {
+    if (refine) invertible_svd_flat<true>(F, thr, sig, U, VT);
+    else invertible_svd_flat<false>(F, thr, sig, U, VT);
+  }
   const double s02 = sig[0] * sig[0], s12 = sig[1] * sig[1], s22 = sig[2] * sig[2];
   const double I1 = s02 + s12 + s22, I3 = s02 * s12 * s22;
   double g0, g1, g2, h0 = 0.0, h5 = 0.0;
@@ -688,10 +691,11 @@ __global__ void __launch_bounds__(kElThreads, kHyperCtas) invhyper_kernel(int ne
                                                               const double* __restrict__ u,
                                                               const double* __restrict__ pre, double thr, double lambda,
                                                               double mu, double* __restrict__ out78,
-                                                              double* __restrict__ out12, const int* __restrict__ perm) {
+                                                              double* __restrict__ out12, const int* __restrict__ perm,
+                                                              bool refine) {
   __shared__ HyperShared sh;
   const int e = blockIdx.x * kElThreads + threadIdx.x;
-  if (e < ne) invhyper_elem<MODE>(e, ne, stvk, tets, X, u, pre, thr, lambda, mu, out78, out12, perm, sh);
+  if (e < ne) invhyper_elem<MODE>(e, ne, stvk, tets, X, u, pre, thr, lambda, mu, out78, out12, perm, refine, sh);
 }
 
 // ---- several scenes per launch: tile j of scene s (directory prefix) is
@@ -715,7 +719,7 @@ __global__ void __launch_bounds__(kElThreads, kHyperCtas) invhyper_batch_kernel(
   const int e = (blockIdx.x - prefix[s]) * kElThreads + threadIdx.x;
   if (e >= D.n_tets) return;
   invhyper_elem<2>(e, D.n_tets, D.kind == OD_MATERIAL_STVK, D.tets, D.X, D.u, D.pre, D.thr, D.lambda, D.mu, D.stage_k,
-                   D.stage_f, nullptr, sh);
+                   D.stage_f, nullptr, true, sh);
 }
 
 // Corotational plastic element (corotationalPlastic.cpp:53-183,
@@ -1166,7 +1170,7 @@ od_status launch_mass(Scene* s) {
   return OD_OK;
 }
 
-od_status launch_eval(Scene* s, bool zero_first) {
+od_status launch_eval(Scene* s, bool zero_first, bool refine) {
   const int T = kElThreads;
   cudaStream_t st = s->ctx->stream;
   if (zero_first && (!s->gat_kptr || s->n_tets == 0)) {
@@ -1187,7 +1191,7 @@ od_status launch_eval(Scene* s, bool zero_first) {
   else
     invhyper_kernel<2><<<nblk(s->n_tets, T), T, 0, st>>>(s->n_tets, s->mat.kind == OD_MATERIAL_STVK, s->tets, s->X, s->u,
                                                           s->pre, s->mat.threshold, s->lambda, s->mu, s->stage_k,
-                                                          s->stage_f, nullptr);
+                                                          s->stage_f, nullptr, refine);
   // 2) assembly: one gather launch; one scatter launch per colour for meshes
   //    whose gather lists do not fit 32-bit indices
   if (s->gat_kptr) {
@@ -1226,7 +1230,7 @@ od_status launch_element_values(Scene* s, double* d_k78, double* d_f12) {
   else
     invhyper_kernel<1><<<nblk(s->n_tets, T), T, 0, st>>>(s->n_tets, s->mat.kind == OD_MATERIAL_STVK, s->tets, s->X, s->u,
                                                           s->pre, s->mat.threshold, s->lambda, s->mu, d_k78, d_f12,
-                                                          s->perm);
+                                                          s->perm, false);
   OD_CUDA(cudaGetLastError());
   return OD_OK;
 }

@@ -504,7 +504,7 @@ void ric_factor(const RicColumns& A, const double* values, double eps, double re
 od_status launch_precompute(Scene* s);
 od_status launch_mass(Scene* s);
 // K, fint at current u
-od_status launch_eval(Scene* s, bool zero_first);
+od_status launch_eval(Scene* s, bool zero_first, bool refine);
 int element_precomputes();   // doubles per element in Scene::pre
 od_status launch_hooke(Scene* s, double youngs, double poisson, double* Kh);  // linear K, reference layout
 // new body force / uniform traction on the facets of the last od_scene_set_loads

@@ -73,7 +73,7 @@ __device__ __forceinline__ float cut_float(double x) {
 // FP32 either); FP64 roots, quotients and transcendental functions are long
 // instruction sequences on the FP64 pipe.  Deviators whose J2 FP32 cannot
 // hold well take the FP64 expressions.
-template <class FT, bool REFINE = false>
+template <class FT, bool REFINE = false, bool ROOTS64 = false>
 __device__ void eig_sym3(const FT* t, FT* vals, FT* vecs) {
   const FT pi = FT(3.141592653589793238462643383279502884);
   const FT s3 = FT(1.7320508075688772935274463415058723669428);
@@ -85,7 +85,7 @@ __device__ void eig_sym3(const FT* t, FT* vals, FT* vecs) {
   const FT J3 = d0 * (d1 * d2 - t[4] * t[4]) + t[1] * (t[4] * t[2] - t[1] * d2) + t[2] * (t[1] * t[4] - d1 * t[2]);
   FT e0;
   bool started = false;
-  if constexpr (REFINE) {
+  if constexpr (REFINE && !ROOTS64) {
     const float j2 = cut_float(J2);
     if (j2 > 1e-24f && j2 < 1e20f) {
       const float pif = 3.14159265358979f, ri = rsqrtf(j2);
@@ -101,7 +101,7 @@ __device__ void eig_sym3(const FT* t, FT* vals, FT* vecs) {
   }
   if (!started) {
     const FT sq = sqrt(J2);
-    const FT cs = (FT(3) * FT(0.5) * s3) * ((J3 / J2) / sq);
+    const FT cs = ROOTS64 ? (FT(3) * FT(0.5) * s3) * (J3 / (J2 * sq)) : (FT(3) * FT(0.5) * s3) * ((J3 / J2) / sq);
     if (isnan(cs) || isinf(cs)) {
       vals[0] = vals[1] = vals[2] = ave;
 #pragma unroll
@@ -109,8 +109,18 @@ __device__ void eig_sym3(const FT* t, FT* vals, FT* vecs) {
       vecs[0] = vecs[4] = vecs[8] = FT(1);
       return;
     }
-    const FT ang = acos(clampv(cs, FT(-1), FT(1))) / FT(3);
-    e0 = (FT(2) / s3) * sq * (ang < pi / FT(6) ? cos(ang) : cos(ang + (FT(2) / FT(3)) * pi));
+    if constexpr (ROOTS64) {
+      const float pif = 3.14159265358979f;
+      const float angf = acosf((float)clampv(cs, FT(-1), FT(1))) / 3.f;
+      const float cf = angf < pif / 6.f ? cosf(angf) : cosf(angf + (2.f / 3.f) * pif);
+      e0 = (FT(2) / s3) * sq * (FT)cf;
+      const FT rdp = FT(1) / (FT(3) * e0 * e0 - J2);
+      e0 -= ((e0 * e0 - J2) * e0 - J3) * rdp;
+      e0 -= ((e0 * e0 - J2) * e0 - J3) * rdp;
+    } else {
+      const FT ang = acos(clampv(cs, FT(-1), FT(1))) / FT(3);
+      e0 = (FT(2) / s3) * sq * (ang < pi / FT(6) ? cos(ang) : cos(ang + (FT(2) / FT(3)) * pi));
+    }
   }
   vals[0] = e0 + ave;
   V3t<FT> r0 = {d0 - e0, t[1], t[2]}, r1 = {t[1], d1 - e0, t[4]}, r2 = {t[2], t[4], d2 - e0};
@@ -550,8 +560,12 @@ __device__ __forceinline__ void coord_system(V3t<FT> v0, V3t<FT>& v1, V3t<FT>& v
 // U from eig(F F^T) made a rotation; V^T = U^T F / sigma with rank-deficient
 // rows completed by cross products; the smallest sigma negated when det V < 0;
 // sigma clamped below by thr.  Outputs U (row-major), VT, sigma.
-template <class FT, bool REFINE = false>
-__device__ void invertible_svd(const FT* F, FT thr, FT* sig, FT* U, FT* VT) {
+// EXACT: every root and sign in FP64.  Returns false, with nothing set, for an F
+// that is too flat for anything else: its smallest eigenvalue carries the
+// largest one's rounding and scales a row of V, so that at a ratio of 1e-8 an
+// ulp of the roots moves the element's stiffness by 1e-8.
+template <class FT, bool REFINE = false, bool EXACT = true>
+__device__ bool invertible_svd(const FT* F, FT thr, FT* sig, FT* U, FT* VT) {
   FT tri[6], ev[3], UT[9];
   tri[0] = F[0] * F[0] + F[1] * F[1] + F[2] * F[2];
   tri[1] = F[3] * F[0] + F[4] * F[1] + F[5] * F[2];
@@ -559,7 +573,11 @@ __device__ void invertible_svd(const FT* F, FT thr, FT* sig, FT* U, FT* VT) {
   tri[3] = F[3] * F[3] + F[4] * F[4] + F[5] * F[5];
   tri[4] = F[6] * F[3] + F[7] * F[4] + F[8] * F[5];
   tri[5] = F[6] * F[6] + F[7] * F[7] + F[8] * F[8];
-  eig_sym3<FT, REFINE>(tri, ev, UT);   // rows e0, e1, e0 x e1: a rotation
+  eig_sym3<FT, REFINE, REFINE && EXACT>(tri, ev, UT);   // rows e0, e1, e0 x e1: a rotation
+  if constexpr (!EXACT) {
+    const FT lo = fmin(ev[0], fmin(ev[1], ev[2])), hi = fmax(ev[0], fmax(ev[1], ev[2]));
+    if (!(lo > FT(0.01) * hi)) return false;
+  }
   // REFINE: sigma = x rsqrt(x), and rsqrt(x) is 1 / sigma for the row scaling
   FT rs[3];
 #pragma unroll
@@ -581,11 +599,16 @@ __device__ void invertible_svd(const FT* F, FT thr, FT* sig, FT* U, FT* VT) {
   switch (cond) {
     case 0: {
       scalerow(0, inv(0)); scalerow(1, inv(1)); scalerow(2, inv(2));
-      // orthonormal rows: det V is 1 or -1 up to rounding
-      float vt[9];
+      bool mirrored;
+      if constexpr (EXACT) {
+        mirrored = det3(VT) < FT(0);
+      } else {   // orthonormal rows: det V is 1 or -1 up to rounding
+        float vt[9];
 #pragma unroll
-      for (int i = 0; i < 9; i++) vt[i] = cut_float(VT[i]);
-      if (det3(vt) < 0.f) {
+        for (int i = 0; i < 9; i++) vt[i] = cut_float(VT[i]);
+        mirrored = det3(vt) < 0.f;
+      }
+      if (mirrored) {
         int sm = ev[0] < ev[1] ? (ev[0] < ev[2] ? 0 : 2) : (ev[1] < ev[2] ? 1 : 2);
         scalerow(sm, FT(-1));
         ev[sm] = -ev[sm];
@@ -610,6 +633,15 @@ __device__ void invertible_svd(const FT* F, FT thr, FT* sig, FT* U, FT* VT) {
   for (int i = 0; i < 3; i++)
 #pragma unroll
     for (int j = 0; j < 3; j++) U[i * 3 + j] = UT[j * 3 + i];
+  return true;
+}
+
+// The same for few elements, out of line.  refine: with the reciprocal roots of
+// the mixed-precision solves' elements, which a flat element tells from the
+// quotients of the FP64 ones'.
+template <bool REFINE>
+__device__ __noinline__ void invertible_svd_flat(const double* F, double thr, double* sig, double* U, double* VT) {
+  invertible_svd<double, REFINE>(F, thr, sig, U, VT);
 }
 
 // PSD projection of a packed symmetric 3x3 (tetelement.cpp:439-465)
