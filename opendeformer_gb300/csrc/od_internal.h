@@ -145,6 +145,8 @@ struct Pcg {
   // solve (both built on first use)
   SliceSys* slice = nullptr;
   MixedSys* mix = nullptr;
+  bool wide_tried = false;
+  struct WidePlan* wide = nullptr;   // the fixed-point PCG of large systems (od_wide.cu); null: not taken
   bool icp_tried = false;
   struct IcPcg* icp = nullptr;  // the one-launch IC(0) PCG's structure (od_ic_pcg.cu); null: not taken
   struct MixIc0* mic = nullptr;  // mixed precision with IC(0) (FP32 factor copy and inner vectors)
@@ -613,6 +615,11 @@ od_status resident_plan(Scene* s);
 void resident_free(ResidentPlan* R);
 od_status resident_solve(Scene* s, const double* d_b, double* d_x, int pkind, double tol, int max_iter, bool x_zero,
                          unsigned long long* prof);
+// the one-launch fixed-point PCG of systems beyond the resident one (od_wide.cu)
+od_status wide_build(Scene* s, WidePlan** out);
+od_status wide_solve(Scene* s, WidePlan* W, const double* d_b, double* d_x, int pkind, double tol, int max_iter, bool x_zero,
+                     unsigned long long* prof);
+void wide_free(WidePlan* W);
 // the one-launch PCG with IC(0) in colour order (od_ic_pcg.cu)
 od_status ic_pcg_build(Scene* s, const std::vector<int>& rp, const std::vector<int>& col, const std::vector<int>& order,
                        const std::vector<int>& cstart, IcPcg** out);

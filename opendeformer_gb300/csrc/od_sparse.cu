@@ -2643,10 +2643,10 @@ od_status pcg_alloc(Scene* s) {
   // a warp would own more than two groups (OD_GB300_PCG_SMEM=0 disables it)
   P.smem_bytes = 0;
   // the one-launch PCG's form: -1 by size and tolerance (at the launch);
-  // OD_GB300_PCG_FORM=standard, =recur or =pipelined forces one
+  // OD_GB300_PCG_FORM=standard, =recur, =pipelined or =wide (od_wide.cu) forces one
   P.recur = -1;
   if (const char* f = std::getenv("OD_GB300_PCG_FORM"))
-    P.recur = std::strcmp(f, "pipelined") == 0 ? 2 : (std::strcmp(f, "recur") == 0 ? 1 : 0);
+    P.recur = std::strcmp(f, "pipelined") == 0 ? 2 : std::strcmp(f, "wide") == 0 ? 3 : (std::strcmp(f, "recur") == 0 ? 1 : 0);
   const char* smem_env = std::getenv("OD_GB300_PCG_SMEM");
   const int nb = s->bsr.nb;
   if (P.coop_grid > 0 && nb > 0 && !(smem_env && smem_env[0] == '0') && (int)s->hbsr_rp.size() == nb + 1) {
@@ -2701,6 +2701,7 @@ void pcg_free(Scene* s) {
   mixed_free(P.mix);
   mixed_ic0_free(P.mic);
   ic_pcg_free(P.icp);
+  wide_free(P.wide);
   slice_free(P.slice);
   sweep_free(P.sweep);
   resident_free(&P.res);
@@ -3416,12 +3417,27 @@ od_status pcg_solve(Scene* s, const double* d_b, double* d_x, const od_solver_pa
     int recur = P.recur >= 0 ? P.recur
                              : (need <= 2 && prm->tol >= 1e-9 ? 2 : (prm->tol >= 1e-10 ? 1 : 0));
     if (recur == 2 && need > 2) recur = 1;
+    // products in fixed point once the vectors are too long for two groups a
+    // warp: an iteration of 237,600 DOFs takes 32 us there and 43 here; at
+    // 161,568 (two groups) 25.4 and 26.7, and a solve's start takes 95 us more
+    const bool wide = P.recur < 0 ? recur == 1 && need > 2 : P.recur == 3;
+    if (recur == 3) recur = 1;
     args[18] = (void*)&recur;
     const bool prof = s->ctx->profiling && s->ctx->ev_pool.size() >= 2;
     const bool phases = prof && s->ctx->profiling >= 2;
     unsigned long long* profp = phases ? P.prof : nullptr;
     args[17] = (void*)&profp;
+    if (wide && !P.wide_tried) {
+      P.wide_tried = true;
+      OD_TRY(wide_build(s, &P.wide));
+    }
     if (prof) OD_CUDA(cudaEventRecord(s->ctx->ev_pool[0], strm));
+    // the recurrence form of systems beyond the chip-resident one
+    if (wide && P.wide) {
+      OD_TRY(wide_solve(s, P.wide, d_b, d_x, pk, prm->tol, prm->max_iter, x_zero, profp));
+      if (prof) OD_CUDA(cudaEventRecord(s->ctx->ev_pool[1], strm));
+      return pcg_finish(s, d_b, d_x, shift, st, true, prof, phases);
+    }
     // chip-resident systems: the pipelined form of od_resident.cu.  Below 1e-9
     // with its true residual verified, and only preconditioned systems of the
     // grid form (more than 5,760 DOFs): in small systems' solves, which run to
