@@ -162,7 +162,7 @@ static od_status batch_build(Batch* B) {
     B->sd_host.push_back(scene_dev(s));
     const int kind = s->mat.kind;
     const bool corot = kind == OD_MATERIAL_COROTATIONAL, plastic = kind == OD_MATERIAL_COROTATIONAL_PLASTIC;
-    const int et = ceil_div(s->n_tets, 128);
+    const int et = ceil_div(s->n_tets, kElThreads);
     const int counts[8] = {ceil_div(s->nvals, kZeroTileValues), ceil_div(s->pcg.n_pad, kZeroTileValues),
                            corot ? et : 0, corot || plastic ? 0 : et, plastic ? et : 0,
                            ceil_div(9LL * s->bsr.nnzb, kExpandTile), ceil_div(s->bsr.nb, kBatchRows),
@@ -179,9 +179,9 @@ static od_status batch_build(Batch* B) {
   auto dir = [&](int d, int size) { return TileDir{B->dirs + (size_t)d * (n + 1), P(d)[n], size}; };
   B->zero_k = dir(0, kZeroTileValues);
   B->zero_f = dir(1, kZeroTileValues);
-  B->corot = dir(2, 128);
-  B->inv = dir(3, 128);
-  B->plastic = dir(4, 128);
+  B->corot = dir(2, kElThreads);
+  B->inv = dir(3, kElThreads);
+  B->plastic = dir(4, kElThreads);
   B->expand = dir(5, kExpandTile);
   B->rows = dir(6, kBatchRows);
   B->dof = dir(7, 256);

@@ -205,13 +205,13 @@ struct ElemOut {
 // 5.0e-16 both).  Exponents outside this window (and NaN and infinities among
 // the factors) take the same sums in FP64.
 // Elements and assembly together, FP64 contraction -> now: Neo-Hookean 98k
-// tets 445 -> 272 us, 655k 2,463 -> 1,375; corotational 416 -> 183 and 2,172 ->
-// 891.  The FP64 unit is about half busy with the decompositions then; what
-// keeps it from more are instruction latency at 16 warps an SM and phases that
-// the warps of one wave pass together.
+// tets 445 -> 256 us, 655k 2,463 -> 1,391; corotational 416 -> 180 and 2,172 ->
+// 896.  The FP64 unit is 40% busy with the decompositions then (506
+// instructions an element); what keeps it from more are instruction latency at
+// 16 warps an SM, waits for constants and instructions, and the last wave of
+// warps (98k tets: 1.26 waves).
 constexpr int kElExpMin = 823, kElExpMax = 1223;   // biased: 2^-200 .. 2^200
-constexpr int kElThreads = 128;
-constexpr int kHyperCtas = 4;   // 128 registers a thread: 16 warps on an SM
+constexpr int kHyperCtas = 8;   // 128 registers a thread: 16 warps on an SM
 
 template <int N>
 __device__ __forceinline__ int max_exp(const double (&v)[N], int e = 0) {
@@ -627,48 +627,63 @@ __device__ __forceinline__ void invhyper_elem(int e, int ne, int stvk, const int
   }
   const double s02 = sig[0] * sig[0], s12 = sig[1] * sig[1], s22 = sig[2] * sig[2];
   const double I1 = s02 + s12 + s22, I3 = s02 * s12 * s22;
-  double g0, g1, g2, h0 = 0.0, h5 = 0.0;
+  // dP/dF non-zeros (tetelement.cpp:357-437).  Neo-Hookean has no derivative
+  // in I2 and one second derivative, in I3; StVK no derivative in I3 and one
+  // second derivative, in I1.  d_ij = I3 g2 / (s_i s_j).
+  const double sc01 = sig[0] * sig[1], sc02 = sig[0] * sig[2], sc12 = sig[1] * sig[2];
+  // I3 / s_i
+  const double qs[3] = {sig[0] * (s12 * s22), sig[1] * (s02 * s22), sig[2] * (s02 * s12)};
+  double al[3], be[3], T[6], de[3];   // de: dE / ds_i
   if (!stvk) {
     const double lI3 = log(I3), rI3 = 1.0 / I3;
-    g0 = 0.5 * mu;
-    g1 = 0.0;
-    g2 = (-0.5 * mu + 0.25 * lambda * lI3) * rI3;
-    h5 = (0.5 * mu + 0.25 * lambda * (1.0 - lI3)) * (rI3 * rI3);
+    const double g0 = 0.5 * mu, g2 = (-0.5 * mu + 0.25 * lambda * lI3) * rI3;
+    const double h5 = (0.5 * mu + 0.25 * lambda * (1.0 - lI3)) * (rI3 * rI3);
+    const double a = 2.0 * g0, h = 4.0 * h5, g = 2.0 * g2;
+    const double d00 = g2 * (s12 * s22), d01 = g2 * (sc01 * s22), d02 = g2 * (sc02 * s12);
+    const double d11 = g2 * (s02 * s22), d12 = g2 * (sc12 * s02), d22 = g2 * (s02 * s12);
+    al[0] = al[1] = al[2] = a;
+    be[0] = -2.0 * d01;
+    be[1] = -2.0 * d02;
+    be[2] = -2.0 * d12;
+    const double h0 = h * qs[0], h1 = h * qs[1], h2 = h * qs[2];
+    T[0] = fma(-2.0, d00, a) + fma(4.0, d00, qs[0] * h0);
+    T[1] = fma(4.0, d01, qs[1] * h0);
+    T[2] = fma(4.0, d02, qs[2] * h0);
+    T[3] = fma(-2.0, d11, a) + fma(4.0, d11, qs[1] * h1);
+    T[4] = fma(4.0, d12, qs[2] * h1);
+    T[5] = fma(-2.0, d22, a) + fma(4.0, d22, qs[2] * h2);
+#pragma unroll
+    for (int i = 0; i < 3; i++) de[i] = fma(g, qs[i], a * sig[i]);
   } else {
-    g0 = 0.25 * lambda * (I1 - 3.0) - 0.5 * mu;
-    g1 = 0.25 * mu;
-    g2 = 0.0;
-    h0 = 0.25 * lambda;
+    const double g0 = 0.25 * lambda * (I1 - 3.0) - 0.5 * mu, g1 = 0.25 * mu;
+    const double a = 2.0 * g0, b = 4.0 * g1, h = lambda;   // h: 4 d2E / dI1^2
+    al[0] = fma(s02 + s12, b, a);
+    al[1] = fma(s02 + s22, b, a);
+    al[2] = fma(s12 + s22, b, a);
+    be[0] = sc01 * b;
+    be[1] = sc02 * b;
+    be[2] = sc12 * b;
+    const double t0 = s02 * b, t1 = s12 * b, t2 = s22 * b, h0 = h * sig[0], h1 = h * sig[1], h2 = h * sig[2];
+    T[0] = fma(2.0, t0, a) + t0 + sig[0] * h0;
+    T[1] = sig[1] * h0;
+    T[2] = sig[2] * h0;
+    T[3] = fma(2.0, t1, a) + t1 + sig[1] * h1;
+    T[4] = sig[2] * h1;
+    T[5] = fma(2.0, t2, a) + t2 + sig[2] * h2;
+    de[0] = sig[0] * (a + t0);
+    de[1] = sig[1] * (a + t1);
+    de[2] = sig[2] * (a + t2);
   }
-  // dP/dF non-zeros (tetelement.cpp:357-437)
-  const double sc01 = sig[0] * sig[1], sc02 = sig[0] * sig[2], sc12 = sig[1] * sig[2];
-  double al[3] = {2.0 * g0 + 4.0 * (s02 + s12) * g1, 2.0 * g0 + 4.0 * (s02 + s22) * g1,
-                  2.0 * g0 + 4.0 * (s12 + s22) * g1};
-  const double a00 = 2.0 * g0 + 8.0 * s02 * g1, a11 = 2.0 * g0 + 8.0 * s12 * g1, a22 = 2.0 * g0 + 8.0 * s22 * g1;
-  // d_ij = I3 g2 / (s_i s_j)
-  const double d00 = g2 * (s12 * s22), d01 = g2 * (sc01 * s22), d02 = g2 * (sc02 * s12);
-  const double d11 = g2 * (s02 * s22), d12 = g2 * (sc12 * s02), d22 = g2 * (s02 * s12);
-  const double b00 = 4.0 * s02 * g1 - 2.0 * d00, b11 = 4.0 * s12 * g1 - 2.0 * d11, b22 = 4.0 * s22 * g1 - 2.0 * d22;
-  double be[3] = {4.0 * sc01 * g1 - 2.0 * d01, 4.0 * sc02 * g1 - 2.0 * d02, 4.0 * sc12 * g1 - 2.0 * d12};
-  // I3 / s_i, and the rows of the invariants' derivatives the Hessians touch:
-  // only H00 (StVK) or H22 (Neo-Hookean) is set
-  const double q0 = sig[0] * (s12 * s22), q1 = sig[1] * (s02 * s22), q2 = sig[2] * (s02 * s12);
-  const double w0[3] = {2.0 * sig[0], 2.0 * sig[1], 2.0 * sig[2]}, w2[3] = {2.0 * q0, 2.0 * q1, 2.0 * q2};
-  auto qf = [&](int i, int j) { return w0[i] * (h0 * w0[j]) + w2[i] * (h5 * w2[j]); };
-  double T[6] = {a00 + b00 + (qf(0, 0) + 4.0 * d00), qf(1, 0) + 4.0 * d01, qf(2, 0) + 4.0 * d02,
-                 a11 + b11 + (qf(1, 1) + 4.0 * d11), qf(2, 1) + 4.0 * d12, a22 + b22 + (qf(2, 2) + 4.0 * d22)};
   psd3<double>(T);
 #pragma unroll
   for (int i = 0; i < 3; i++) psd2<double>(al[i], be[i]);
   const double vol = pre[(size_t)kPreVol * ne + e];
   const ElemOut<MODE> out(e, out78, out12, perm);
-  const double qs[3] = {q0, q1, q2};
   double dvt[9];
 #pragma unroll
   for (int i = 0; i < 3; i++) {
-    const double de = 2.0 * g0 * sig[i] + 4.0 * g1 * sig[i] * sig[i] * sig[i] + 2.0 * g2 * qs[i];
 #pragma unroll
-    for (int j = 0; j < 3; j++) dvt[i * 3 + j] = de * VT[i * 3 + j];
+    for (int j = 0; j < 3; j++) dvt[i * 3 + j] = de[i] * VT[i * 3 + j];
   }
   stress_forces<MODE>(U, dvt, Di, vol, out);
   hyper_stiffness<MODE>(U, VT, Di, T, al, be, vol, sh, out);
@@ -699,7 +714,7 @@ __global__ void __launch_bounds__(kElThreads, kHyperCtas) invhyper_kernel(int ne
 }
 
 // ---- several scenes per launch: tile j of scene s (directory prefix) is
-// its elements [128 j, 128 j + 128); every scene's values land in its own
+// its elements [kElThreads j, kElThreads (j + 1)); every scene's values land in its own
 // staging arrays
 __global__ void __launch_bounds__(kElThreads) corot_batch_kernel(int n_sc, const int* __restrict__ prefix,
                                                                  const SceneDev* __restrict__ sd) {
@@ -815,7 +830,7 @@ __global__ void __launch_bounds__(kElThreads) plastic_batch_kernel(int n_sc, con
   __shared__ int2 sa[12][kElThreads];
   const int s = dir_scene(prefix, n_sc, blockIdx.x);
   const SceneDev& D = sd[s];
-  const int e = (blockIdx.x - prefix[s]) * 128 + threadIdx.x;
+  const int e = (blockIdx.x - prefix[s]) * kElThreads + threadIdx.x;
   if (e >= D.n_tets) return;
   plastic_elem<2>(e, D.n_tets, D.tets, D.X, D.u, D.pre, D.thr, D.lambda, D.mu, D.yield, D.creep, D.max_plastic,
                   D.plastic, D.stage_k, D.stage_f, nullptr, sa);
@@ -1296,15 +1311,15 @@ od_status launch_eval_batch(Ctx* ctx, int n_sc, const SceneDev* sd, const TileDi
   }
   if (corot.tiles > 0) {
     ctx->launches++;
-    corot_batch_kernel<<<corot.tiles, 128, 0, st>>>(n_sc, corot.prefix, sd);
+    corot_batch_kernel<<<corot.tiles, kElThreads, 0, st>>>(n_sc, corot.prefix, sd);
   }
   if (inv.tiles > 0) {
     ctx->launches++;
-    invhyper_batch_kernel<<<inv.tiles, 128, 0, st>>>(n_sc, inv.prefix, sd);
+    invhyper_batch_kernel<<<inv.tiles, kElThreads, 0, st>>>(n_sc, inv.prefix, sd);
   }
   if (plastic.tiles > 0) {
     ctx->launches++;
-    plastic_batch_kernel<<<plastic.tiles, 128, 0, st>>>(n_sc, plastic.prefix, sd);
+    plastic_batch_kernel<<<plastic.tiles, kElThreads, 0, st>>>(n_sc, plastic.prefix, sd);
   }
   if (gathered) {
     if (gather.tiles > 0) {

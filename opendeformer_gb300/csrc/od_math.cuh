@@ -132,17 +132,18 @@ __device__ void eig_sym3(const FT* t, FT* vals, FT* vecs) {
     l1 = sqrt(l1);
     l2 = sqrt(l2);
   }
+  // the longest row, then the two others in order: choices of values, one
+  // normalisation each -- the lanes of a warp choose differently, and what
+  // each choice computed on its own all of them would pay for
   auto norm0 = [&](V3t<FT> v, FT l) { return REFINE ? v_scale(v, rsqrt(l)) : v_div(v, l); };
-  V3t<FT> s0, t1, t2;
-  if (l0 > l1) {
-    if (l0 > l2) { s0 = norm0(r0, l0); t1 = v_sub(r1, v_scale(s0, v_dot(s0, r1))); t2 = v_sub(r2, v_scale(s0, v_dot(s0, r2))); }
-    else { s0 = norm0(r2, l2); t1 = v_sub(r0, v_scale(s0, v_dot(s0, r0))); t2 = v_sub(r1, v_scale(s0, v_dot(s0, r1))); }
-  } else {
-    if (l1 > l2) { s0 = norm0(r1, l1); t1 = v_sub(r0, v_scale(s0, v_dot(s0, r0))); t2 = v_sub(r2, v_scale(s0, v_dot(s0, r2))); }
-    else { s0 = norm0(r2, l2); t1 = v_sub(r0, v_scale(s0, v_dot(s0, r0))); t2 = v_sub(r1, v_scale(s0, v_dot(s0, r1))); }
-  }
+  auto pick = [](bool c, V3t<FT> a, V3t<FT> b) { return V3t<FT>{c ? a.x : b.x, c ? a.y : b.y, c ? a.z : b.z}; };
+  const bool by0 = l0 > l1 && l0 > l2, by1 = !(l0 > l1) && l1 > l2;
+  const V3t<FT> s0 = norm0(pick(by0, r0, pick(by1, r1, r2)), by0 ? l0 : by1 ? l1 : l2);
+  const V3t<FT> p1 = pick(by0, r1, r0), p2 = pick(by0 || by1, r2, r1);
+  const V3t<FT> t1 = v_sub(p1, v_scale(s0, v_dot(s0, p1))), t2 = v_sub(p2, v_scale(s0, v_dot(s0, p2)));
   FT t1l = v_len2(t1), t2l = v_len2(t2);
-  V3t<FT> s1 = t1l > t2l ? unit(t1, t1l) : unit(t2, t2l);
+  const bool first = t1l > t2l;
+  V3t<FT> s1 = unit(pick(first, t1, t2), first ? t1l : t2l);
   V3t<FT> ev0 = v_cross(s0, s1);
   vecs[0] = ev0.x; vecs[1] = ev0.y; vecs[2] = ev0.z;
   auto mulm = [&](V3t<FT> v) {
@@ -158,7 +159,8 @@ __device__ void eig_sym3(const FT* t, FT* vals, FT* vecs) {
   V3t<FT> u0 = v_cross(v_sub(m0, v_scale(s0, e1)), ev0);
   V3t<FT> u1 = v_cross(v_sub(m1, v_scale(s1, e1)), ev0);
   FT u0l = v_len2(u0), u1l = v_len2(u1);
-  V3t<FT> ev1 = (u0l != FT(0)) ? (u0l > u1l ? unit(u0, u0l) : unit(u1, u1l)) : s0;
+  const bool longer = u0l > u1l;
+  const V3t<FT> ev1 = pick(u0l != FT(0), unit(pick(longer, u0, u1), longer ? u0l : u1l), s0);
   vecs[3] = ev1.x; vecs[4] = ev1.y; vecs[5] = ev1.z;
   V3t<FT> ev2 = v_cross(ev0, ev1);
   vecs[6] = ev2.x; vecs[7] = ev2.y; vecs[8] = ev2.z;
@@ -579,7 +581,7 @@ __device__ bool invertible_svd(const FT* F, FT thr, FT* sig, FT* U, FT* VT) {
     if (!(lo > FT(0.01) * hi)) return false;
   }
   // REFINE: sigma = x rsqrt(x), and rsqrt(x) is 1 / sigma for the row scaling
-  FT rs[3];
+  FT rs[3] = {};
 #pragma unroll
   for (int i = 0; i < 3; i++) {
     if constexpr (REFINE) {
