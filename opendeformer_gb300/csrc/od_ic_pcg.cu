@@ -944,6 +944,7 @@ od_status ic_pcg_solve(Scene* s, IcPcg* I, const double* d_b, double* d_x, doubl
   OD_CUDA(cudaMemsetAsync(I->ctr, 0, sizeof(unsigned) * (4 * kIpCtr + kIpShifts), st));
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute at;
+  s->ctx->sweep_levels = 2 * I->nc;
   void* args[] = {(void*)&a};
   ic_pcg_config(I->factor_grid, I->factor_smem, false, st, &cfg, &at);
   OD_KL(s);
