@@ -307,6 +307,7 @@ struct Ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
   int num_sms = 0;
+  bool host_tables = false;           // the device reads pageable host memory through the host's page tables
   // counters
   long long launches = 0;
   long long host_syncs = 0;

@@ -2507,7 +2507,7 @@ static od_status ic0_one_launch(Scene* s) {
   if (P.icp_tried) return OD_OK;
   P.icp_tried = true;
   const char* order = std::getenv("OD_GB300_IC0_ORDER");
-  if (std::getenv("OD_GB300_IC0_FACTOR") || std::getenv("OD_GB300_IC0_SWEEP") ||
+  if (P.disable_persistent || std::getenv("OD_GB300_IC0_FACTOR") || std::getenv("OD_GB300_IC0_SWEEP") ||
       (order && std::strcmp(order, "natural") == 0))
     return OD_OK;
   const int nb = s->bsr.nb;
