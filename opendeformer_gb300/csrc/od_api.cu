@@ -32,6 +32,15 @@ od_status sync_stream(Scene* s) {
   return OD_OK;
 }
 
+// p is host memory that kernels may use as it is
+static bool host_reached(const Ctx* ctx, const void* p) {
+  cudaPointerAttributes at{};
+  const bool ok = ctx->host_tables && cudaPointerGetAttributes(&at, p) == cudaSuccess &&
+                  (at.type == cudaMemoryTypeUnregistered || at.type == cudaMemoryTypeHost);
+  cudaGetLastError();
+  return ok;
+}
+
 // Several arrays of n doubles between host and device (null: none).  Where the
 // device reads the host's page tables a kernel copies them all at once, from or
 // to pageable memory: three arrays of 20,000 take 13 us in and 12 us out, one
@@ -50,17 +59,13 @@ __global__ void copy_arrays_kernel(const __grid_constant__ CopyArrays c, int n) 
 static od_status copy_arrays(Scene* s, const double* const (&src)[3], double* const (&dst)[3], int n, cudaMemcpyKind kind) {
   CopyArrays c{};
   int count = 0;
-  bool direct = s->ctx->host_tables;
+  bool direct = true;
   for (int k = 0; k < 3; k++) {
     if (!src[k] || !dst[k]) continue;
     c.src[count] = src[k];
     c.dst[count++] = dst[k];
-    cudaPointerAttributes at{};
-    const void* host = kind == cudaMemcpyHostToDevice ? (const void*)src[k] : (const void*)dst[k];
-    direct = direct && cudaPointerGetAttributes(&at, host) == cudaSuccess &&
-             (at.type == cudaMemoryTypeUnregistered || at.type == cudaMemoryTypeHost);
+    direct = direct && host_reached(s->ctx, kind == cudaMemcpyHostToDevice ? src[k] : dst[k]);
   }
-  cudaGetLastError();
   if (n <= 0) return OD_OK;
   if (direct && count > 1) {
     OD_KL(s);
@@ -525,9 +530,13 @@ od_status od_scene_evaluate(od_scene* scene, double* values, double* f_int) {
   OD_CHECK_ARG(scene, "od_scene_evaluate: scene is NULL");
   Scene* s = &scene->s;
   OD_CUDA(cudaSetDevice(s->ctx->device));
-  OD_TRY(launch_eval(s, true, false));
-  if (values) OD_CUDA(cudaMemcpyAsync(values, s->K, sizeof(double) * s->nvals, cudaMemcpyDeviceToHost, s->ctx->stream));
-  if (f_int) OD_CUDA(cudaMemcpyAsync(f_int, s->fint, sizeof(double) * s->dofs, cudaMemcpyDeviceToHost, s->ctx->stream));
+  // where the device reaches the host's arrays the assembly writes them as it
+  // goes, instead of two copies after it
+  double* hk = s->gat_kptr && values && host_reached(s->ctx, values) ? values : nullptr;
+  double* hf = s->gat_kptr && f_int && host_reached(s->ctx, f_int) ? f_int : nullptr;
+  OD_TRY(launch_eval(s, true, false, hk, hf));
+  if (values && !hk) OD_CUDA(cudaMemcpyAsync(values, s->K, sizeof(double) * s->nvals, cudaMemcpyDeviceToHost, s->ctx->stream));
+  if (f_int && !hf) OD_CUDA(cudaMemcpyAsync(f_int, s->fint, sizeof(double) * s->dofs, cudaMemcpyDeviceToHost, s->ctx->stream));
   OD_TRY(sync_stream(s));
   return OD_OK;
 }
@@ -568,9 +577,13 @@ od_status od_scene_spmdv(od_scene* scene, const double* values, const double* x,
   OD_CUDA(cudaSetDevice(s->ctx->device));
   OD_CUDA(cudaMemcpyAsync(s->work_vals, values, sizeof(double) * s->nvals, cudaMemcpyHostToDevice, st));
   OD_CUDA(cudaMemcpyAsync(s->tmp, x, sizeof(double) * s->dofs, cudaMemcpyHostToDevice, st));
-  OD_CUDA(cudaMemcpyAsync(s->tmp2, y, sizeof(double) * s->dofs, cudaMemcpyHostToDevice, st));
-  OD_TRY(launch_spmv_lower(s, s->work_vals, 1.0, s->tmp, nullptr, 0.0, nullptr, nullptr, 0.0, nullptr, s->tmp2, true));
-  OD_CUDA(cudaMemcpyAsync(y, s->tmp2, sizeof(double) * s->dofs, cudaMemcpyDeviceToHost, st));
+  // y, read and written once, stays where it is if the device reaches it (and
+  // has no padding)
+  const bool there = s->dofs == s->pcg.n_pad && host_reached(s->ctx, y);
+  double* acc = there ? y : s->tmp2;
+  if (!there) OD_CUDA(cudaMemcpyAsync(acc, y, sizeof(double) * s->dofs, cudaMemcpyHostToDevice, st));
+  OD_TRY(launch_spmv_lower(s, s->work_vals, 1.0, s->tmp, nullptr, 0.0, nullptr, nullptr, 0.0, nullptr, acc, true));
+  if (!there) OD_CUDA(cudaMemcpyAsync(y, acc, sizeof(double) * s->dofs, cudaMemcpyDeviceToHost, st));
   OD_TRY(sync_stream(s));
   return OD_OK;
 }

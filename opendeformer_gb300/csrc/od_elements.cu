@@ -867,29 +867,34 @@ __device__ __forceinline__ void gather_one(long long i, int nk, const int* __res
                                            const int* __restrict__ ksrc, const double* __restrict__ k78,
                                            double* __restrict__ K, int nf, const int* __restrict__ fptr,
                                            const int* __restrict__ fsrc, const double* __restrict__ f12,
-                                           double* __restrict__ fint, int accumulate) {
+                                           double* __restrict__ fint, int accumulate, double* host_k = nullptr,
+                                           double* host_f = nullptr, int host_nf = 0) {
   const int* ptr = kptr;
   const int* src = ksrc;
   const double* val = k78;
   double* out = K;
+  double* host = host_k;
   if (i >= nk) {
     i -= nk;
     if (i >= nf) return;
     ptr = fptr; src = fsrc; val = f12; out = fint;
+    host = i < host_nf ? host_f : nullptr;
   }
   const int j1 = ptr[i + 1];
   double acc = accumulate ? out[i] : 0.0;
   for (int j = ptr[i]; j < j1; j++) acc += val[src[j]];
   out[i] = acc;
+  if (host) host[i] = acc;
 }
 
 __global__ void __launch_bounds__(256) gather_kernel(int nk, const int* __restrict__ kptr,
                                                      const int* __restrict__ ksrc, const double* __restrict__ k78,
                                                      double* __restrict__ K, int nf, const int* __restrict__ fptr,
                                                      const int* __restrict__ fsrc, const double* __restrict__ f12,
-                                                     double* __restrict__ fint, int accumulate) {
+                                                     double* __restrict__ fint, int accumulate, double* host_k = nullptr,
+                                                     double* host_f = nullptr, int host_nf = 0) {
   gather_one((long long)blockIdx.x * blockDim.x + threadIdx.x, nk, kptr, ksrc, k78, K, nf, fptr, fsrc, f12, fint,
-             accumulate);
+             accumulate, host_k, host_f, host_nf);
 }
 
 // multi-scene scatter of colour c: tile j of scene s covers the colour's
@@ -1185,7 +1190,7 @@ od_status launch_mass(Scene* s) {
   return OD_OK;
 }
 
-od_status launch_eval(Scene* s, bool zero_first, bool refine) {
+od_status launch_eval(Scene* s, bool zero_first, bool refine, double* host_k, double* host_f) {
   const int T = kElThreads;
   cudaStream_t st = s->ctx->stream;
   if (zero_first && (!s->gat_kptr || s->n_tets == 0)) {
@@ -1214,7 +1219,7 @@ od_status launch_eval(Scene* s, bool zero_first, bool refine) {
     if (nd == 0) return OD_OK;
     OD_KL(s);
     gather_kernel<<<nblk(nd, 256), 256, 0, st>>>(s->nvals, s->gat_kptr, s->gat_ksrc, s->stage_k, s->K, s->pcg.n_pad,
-                                                 s->gat_fptr, s->gat_fsrc, s->stage_f, s->fint, zero_first ? 0 : 1);
+                                                 s->gat_fptr, s->gat_fsrc, s->stage_f, s->fint, zero_first ? 0 : 1, host_k, host_f, s->dofs);
     OD_CUDA(cudaGetLastError());
     return OD_OK;
   }

@@ -510,8 +510,9 @@ void ric_factor(const RicColumns& A, const double* values, double eps, double re
 constexpr int kElThreads = 64;
 od_status launch_precompute(Scene* s);
 od_status launch_mass(Scene* s);
-// K, fint at current u
-od_status launch_eval(Scene* s, bool zero_first, bool refine);
+// K, fint at current u; with host_k and host_f (scenes with gather lists only,
+// memory the device reaches) the assembly also writes them there: see od_api.cu
+od_status launch_eval(Scene* s, bool zero_first, bool refine, double* host_k = nullptr, double* host_f = nullptr);
 int element_precomputes();   // doubles per element in Scene::pre
 od_status launch_hooke(Scene* s, double youngs, double poisson, double* Kh);  // linear K, reference layout
 // new body force / uniform traction on the facets of the last od_scene_set_loads
