@@ -2,6 +2,7 @@
 // integrator entry points and the step drivers.
 #include <algorithm>
 #include <cmath>
+#include <cstdint>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -32,10 +33,10 @@ od_status sync_stream(Scene* s) {
   return OD_OK;
 }
 
-// p is host memory that kernels may use as it is
+// p is host memory that kernels may use as it is (copies take any alignment)
 static bool host_reached(const Ctx* ctx, const void* p) {
   cudaPointerAttributes at{};
-  const bool ok = ctx->host_tables && cudaPointerGetAttributes(&at, p) == cudaSuccess &&
+  const bool ok = ctx->host_tables && reinterpret_cast<uintptr_t>(p) % alignof(double) == 0 && cudaPointerGetAttributes(&at, p) == cudaSuccess &&
                   (at.type == cudaMemoryTypeUnregistered || at.type == cudaMemoryTypeHost);
   cudaGetLastError();
   return ok;
@@ -65,6 +66,8 @@ static od_status copy_arrays(Scene* s, const double* const (&src)[3], double* co
     c.src[count] = src[k];
     c.dst[count++] = dst[k];
     direct = direct && host_reached(s->ctx, kind == cudaMemcpyHostToDevice ? src[k] : dst[k]);
+    for (int q = 0; q + 1 < count; q++)   // arrays that overlap: the last copy is what stays
+      direct = direct && (c.dst[q] + n <= dst[k] || dst[k] + n <= c.dst[q]);
   }
   if (n <= 0) return OD_OK;
   if (direct && count > 1) {

@@ -27,6 +27,13 @@ def test_state_round_trip(dims):
     s.set_state(v, None, d)
     for got, want in zip(s.state(), (bits[1], bits[0], bits[0])):
         assert np.array_equal(got.view(np.uint64), want)
+    # doubles at odd addresses: by copies, as any alignment
+    odd = [np.frombuffer(bytearray(8 * s.dofs + 4), dtype=np.float64, offset=4) for _ in range(3)]
+    for to, x in zip(odd, (v, a, d)):
+        to[:] = x
+    s.set_state(*odd)
+    for got, want in zip(s.state(), (bits[1], bits[2], bits[0])):
+        assert np.array_equal(got.view(np.uint64), want)
     torch = pytest.importorskip("torch")
     pinned = [torch.from_numpy(x.copy()).pin_memory().numpy() for x in (a, d, v)]
     s.set_state(*pinned)
@@ -37,7 +44,7 @@ def test_state_round_trip(dims):
 @pytest.mark.parametrize("drop", [0, 1])
 @pytest.mark.parametrize("dims", [(1, 1, 1), (5, 4, 3)])
 def test_evaluate_and_product_into_host_memory(dims, drop):
-    """Touched, untouched and pinned arrays receive the same bits; with `drop` a constrained DOF less, so that the last
+    """Touched, untouched, pinned and misaligned arrays receive the same bits; with `drop` a constrained DOF less, so that the last
     block row is padded and y goes by copies.  The product against the oracle's, within its rounding of some 20 terms."""
     import ctypes as C
 
@@ -54,7 +61,8 @@ def test_evaluate_and_product_into_host_memory(dims, drop):
     K, f = s.evaluate()
     p = lambda a: a.ctypes.data_as(C.POINTER(C.c_double))
     L = api.load_library()
-    for make in (lambda n: np.full(n, 7.0), lambda n: np.empty(n), lambda n: torch.empty(n, dtype=torch.float64).pin_memory().numpy()):
+    odd = lambda n: np.frombuffer(bytearray(8 * n + 4), dtype=np.float64, offset=4)
+    for make in (lambda n: np.full(n, 7.0), np.empty, odd, lambda n: torch.empty(n, dtype=torch.float64).pin_memory().numpy()):
         k2, f2 = make(s.n_values), make(s.dofs)
         assert L.od_scene_evaluate(s.h, p(k2), p(f2)) == 0
         assert np.array_equal(k2, K) and np.array_equal(f2, f)
