@@ -3456,12 +3456,14 @@ od_status pcg_solve(Scene* s, const double* d_b, double* d_x, const od_solver_pa
       return pcg_finish(s, d_b, d_x, shift, st, true, prof, phases);
     }
     // chip-resident systems: the pipelined form of od_resident.cu.  Below 1e-9
-    // with its true residual verified, and only preconditioned systems of the
-    // grid form (more than 5,760 DOFs): in small systems' solves, which run to
-    // their dimension, and unpreconditioned ones the residuals part so far
-    // that going on from the true one takes more iterations (129 against 123
-    // without a preconditioner, 1.5% over 20 steps of 105 DOFs)
-    const bool verify = P.recur < 0 && recur == 1 && pk != OD_PRECOND_NONE && !P.res.cluster;
+    // with its true residual verified, and only preconditioned systems of 240
+    // DOFs and more: in solves that run to their dimension, and unpreconditioned
+    // ones, the residuals part so far that going on from the true one takes more
+    // iterations (129 against 123 without a preconditioner, 1.5% over 20 steps of
+    // 105 DOFs; 0.7% at 252 DOFs, 0.1% at 1,260).  A call of 200 iterations at
+    // 1e-10: 252 DOFs 1,950 -> 480 us, 1,260 2,500 -> 680, 4,860 2,760 -> 1,040
+    constexpr int kVerifyRows = 80;
+    const bool verify = P.recur < 0 && recur == 1 && pk != OD_PRECOND_NONE && nb >= kVerifyRows;
     if (P.res.warps > 0 && (recur == 2 || verify)) {
       OD_TRY(resident_solve(s, d_b, d_x, pk, prm->tol, prm->max_iter, x_zero, profp));
       if (prof) OD_CUDA(cudaEventRecord(s->ctx->ev_pool[1], strm));
