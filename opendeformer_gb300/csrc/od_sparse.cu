@@ -3456,14 +3456,15 @@ od_status pcg_solve(Scene* s, const double* d_b, double* d_x, const od_solver_pa
       return pcg_finish(s, d_b, d_x, shift, st, true, prof, phases);
     }
     // chip-resident systems: the pipelined form of od_resident.cu.  Below 1e-9
-    // with its true residual verified, and only preconditioned systems of 240
-    // DOFs and more: in solves that run to their dimension, and unpreconditioned
-    // ones, the residuals part so far that going on from the true one takes more
-    // iterations (129 against 123 without a preconditioner, 1.5% over 20 steps of
-    // 105 DOFs; 0.7% at 252 DOFs, 0.1% at 1,260).  A call of 200 iterations at
-    // 1e-10: 252 DOFs 1,950 -> 480 us, 1,260 2,500 -> 680, 4,860 2,760 -> 1,040
-    constexpr int kVerifyRows = 80;
-    const bool verify = P.recur < 0 && recur == 1 && pk != OD_PRECOND_NONE && nb >= kVerifyRows;
+    // with its true residual verified, from the sizes on at which going on from
+    // the true residual takes at most about 1% more iterations (solves that run to
+    // their dimension part from it: preconditioned 1.5% at 105 DOFs, 0.7% at 252,
+    // 0.1% at 1,260; without a preconditioner 2.7% at 252, 1.1% at 720, 0.4% at
+    // 1,260, none at 12,000).  A call of 200 iterations at 1e-10: 252 DOFs 1,950
+    // -> 480 us, 1,260 2,500 -> 680, 4,860 2,760 -> 1,040; 260 iterations without a
+    // preconditioner 720 DOFs 3,150 -> 760, 12,870 3,500 -> 1,570
+    const int verify_rows = pk == OD_PRECOND_NONE ? 240 : 80;
+    const bool verify = P.recur < 0 && recur == 1 && nb >= verify_rows;
     if (P.res.warps > 0 && (recur == 2 || verify)) {
       OD_TRY(resident_solve(s, d_b, d_x, pk, prm->tol, prm->max_iter, x_zero, profp));
       if (prof) OD_CUDA(cudaEventRecord(s->ctx->ev_pool[1], strm));
