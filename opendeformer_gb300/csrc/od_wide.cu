@@ -502,10 +502,12 @@ __device__ __forceinline__ void wide_body(const WideArgs& P, WideShared& sh, dou
     }
     return fx;
   };
-  // z = M^-1 r, its digits at the scale E, r.z and r.r of this thread's entries
+  // z = M^-1 r, r.z and r.r of this thread's entries; digits: z's at the scale E
+  // too.  Only where a sync lies behind the last product: other CTAs may still be
+  // gathering what P.zd holds (at the start x's digits)
   double rz = 0.0, rr = 0.0;
   int ez = 0;
-  auto precondition = [&]() {
+  auto precondition = [&](bool digits) {
     rz = rr = 0.0;
     ez = 0;
     for (int i = threadIdx.x; i < own; i += kWdThreads) {
@@ -518,7 +520,7 @@ __device__ __forceinline__ void wide_body(const WideArgs& P, WideShared& sh, dou
         z = I[i] * r;
       }
       Z[i] = z;
-      P.zd[kWdLanes * (size_t)c0 + i] = fx_digits(z, E);
+      if (digits) P.zd[kWdLanes * (size_t)c0 + i] = fx_digits(z, E);
       ez = max(ez, fx_biased_exp(z));
       rz = fma(r, z, rz);
       rr = fma(r, r, rr);
@@ -549,7 +551,7 @@ __device__ __forceinline__ void wide_body(const WideArgs& P, WideShared& sh, dou
     const double b = d >= 0 ? P.b[d] : 0.0;
     bb = fma(b, b, bb);
   }
-  precondition();
+  precondition(false);
   if (!wide_sums<3>(P, sh, rz, rr, bb, ez, ++es)) return;
   rz = sh.tot[0];
   rr = sh.tot[1];
@@ -577,7 +579,7 @@ __device__ __forceinline__ void wide_body(const WideArgs& P, WideShared& sh, dou
     __syncthreads();
     E = e - 1021;
     ready = true;
-    precondition();
+    precondition(true);
     stamp(2);
     if (!wide_sums<2>(P, sh, rz, rr, 0.0, ez, ++es)) return;
     stamp(3);
