@@ -116,7 +116,11 @@ struct ResidentShared {
   int cep[2][kRgCluster];           // and largest exponents
   double ab[2];                 // alpha, beta
   double tot[3];                // the last grid-wide sums
-  int stop, status, iter;
+  // by the parity of the round: the sync warp reads its round's word while the
+  // first sum warp may be writing the next round's.  That one's next write of
+  // the same word lies behind a kBarStep that the sync warp takes part in
+  int stop[2];
+  int status, iter;
   int emax;                     // the last vector's largest biased exponent
   int ew[kRgMaxWarps];          // its worker warps'
   int fail;                     // a wait ran out
@@ -557,7 +561,7 @@ __device__ __forceinline__ void resident_body(const ResidentArgs& P, unsigned ch
       x = fma(alpha, p, x);
       bar_sync(kBarStep, all);
       stamp(3);
-      if (sh.stop) break;
+      if (sh.stop[par]) break;
       const int top = sh.emax - 1022;          // 2^top is above m
       if (valid && (top > E || top < E - kFxSlack || !row_fx))
         n = row_product_m<CL>(P.A + 9 * (size_t)kb, cols, ke - kb, t10, rsub, P.m[par], (2 + par) * mrow);
@@ -576,7 +580,7 @@ __device__ __forceinline__ void resident_body(const ResidentArgs& P, unsigned ch
     }
   } else if (w == W) {
 #pragma unroll 1
-    do {
+    for (int par = 0;; par ^= 1) {
       bar_sync(kBarM, nt + 32);
       epoch++;
       const int e = sync_grid<CL>(P, sh, epoch & 1, epoch, [&] {
@@ -586,7 +590,8 @@ __device__ __forceinline__ void resident_body(const ResidentArgs& P, unsigned ch
       if (lane == 0) sh.emax = e;
       __syncwarp();
       bar_sync(kBarStep, all);
-    } while (!sh.stop);
+      if (sh.stop[par]) break;
+    }
   } else {
     // sum warp j takes dot product j; the first forms the step lengths
     const int j = w - W - 1;
@@ -602,7 +607,7 @@ __device__ __forceinline__ void resident_body(const ResidentArgs& P, unsigned ch
       if (j > 0) {
         bar_arrive(kBarTot, 96);
         bar_sync(kBarStep, all);
-        if (sh.stop) break;
+        if (sh.stop[it & 1]) break;
         continue;
       }
       // beta = gamma / gamma_prev, alpha = gamma / den with den = delta -
@@ -628,7 +633,7 @@ __device__ __forceinline__ void resident_body(const ResidentArgs& P, unsigned ch
       if (lane == 0) {
         sh.ab[0] = alpha;
         sh.ab[1] = beta;
-        sh.stop = stop;
+        sh.stop[it & 1] = stop;
         if (stop) {
           sh.status = status;
           sh.iter = it;
@@ -636,7 +641,7 @@ __device__ __forceinline__ void resident_body(const ResidentArgs& P, unsigned ch
       }
       __syncwarp();
       bar_sync(kBarStep, all);
-      if (stop) break;
+      if (sh.stop[it & 1]) break;   // lane 0's word: the lanes' reads of fail may differ
       gam_inv = 1.0 / t;
       den_k = den * gam_inv * gam_inv;
     }
@@ -678,7 +683,7 @@ __global__ void __launch_bounds__(32 * (MAXW + kRgServe), 1) pcg_resident_kernel
   __shared__ ResidentShared sh;
   if (threadIdx.x == 0) {
     sh.fail = 0;
-    sh.stop = 0;
+    sh.stop[0] = sh.stop[1] = 0;
     sh.status = OD_OK;
     for (int k = 0; k < kPcgProfSlots; k++) sh.prof[k] = 0;
     if constexpr (CL)
