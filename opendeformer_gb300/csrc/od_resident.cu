@@ -74,6 +74,7 @@ struct ResidentArgs {
   int nb, ngroups, warps;       // block rows; groups; worker warps per CTA
   const int* rp;
   const int* col;
+  const int* diag;              // every block row's diagonal block
   const double* A;              // full BSR
   const double* b;
   double* x;
@@ -296,8 +297,8 @@ __device__ __noinline__ double row_product_m(const double* A, const unsigned* co
 }
 
 // One block row's matrix steps as digits, by its three lanes (r: this lane's
-// row of the blocks, t: the block row's place in the group): the values, then
-// the scale of the row's sum of magnitudes (from the leading 21 bits of each,
+// row of the blocks, t: the block row's place in the group): the values over
+// their columns' powers of two (fx_column_exp), then the scale of the row's sum of magnitudes (from the leading 21 bits of each,
 // rounded up), then the digits in place.  A column entry is the gathered row's
 // byte offset, in the cluster form its shared-memory address (mx: this CTA's
 // first row).  Returns the scale, kFxNone for a row without one (its products
@@ -310,14 +311,15 @@ __device__ __noinline__ int stage_rows(const ResidentArgs& P, double* raw, unsig
   for (int j = 0; j < steps; j++) {
     const bool in = kb + j < ke;
     const double* a = P.A + 9 * (size_t)(kb + j) + 3 * r;
+    const int cb = in ? P.col[kb + j] : min(row, P.nb - 1);
+    const double* d = P.A + 9 * (size_t)P.diag[cb];
 #pragma unroll
     for (int c = 0; c < 3; c++) {
-      const double v = in ? a[c] : 0.0;
+      const double v = in ? fx_times_pow2(a[c], -fx_column_exp(d[4 * c])) : 0.0;
       raw[rg_value(j, r, 3 * t + c)] = v;
       em = max(em, fx_biased_exp(v));
     }
     if (r == 0) {
-      const int cb = in ? P.col[kb + j] : min(row, P.nb - 1);
       unsigned at = kRgRowBytes * cb;
       if constexpr (CL) {
         const int g = cb / kRgRows, G = gridDim.x, c = ((g + 1) * G - 1) / P.ngroups;
@@ -413,6 +415,7 @@ __device__ __forceinline__ void resident_body(const ResidentArgs& P, unsigned ch
     __syncwarp();
   }
   const bool row_fx = ea != kFxNone;
+  const int kc = valid ? fx_column_exp(P.A[9 * (size_t)P.diag[row] + 4 * rsub]) : 0;   // of this lane's entry
   double pm0 = 1.0, pm1 = 0.0, pm2 = 0.0;
   if (valid) {
     if (P.pkind == OD_PRECOND_JACOBI) {
@@ -503,7 +506,7 @@ __device__ __forceinline__ void resident_body(const ResidentArgs& P, unsigned ch
     u = precond(r);
     if (valid) P.u0[i] = u;
     vals[threadIdx.x] = valid ? bv * bv : 0.0;
-    const int e = __reduce_max_sync(0xffffffffu, valid ? fx_biased_exp(u) : 0);
+    const int e = __reduce_max_sync(0xffffffffu, valid ? fx_biased_exp(u, kc) : 0);
     if (lane == 0) sh.ew[w] = e;
   }
   if (!full_sync<CL>(P, sh, vals, epoch)) return;
@@ -522,8 +525,8 @@ __device__ __forceinline__ void resident_body(const ResidentArgs& P, unsigned ch
   };
   stamp(-1);
   const int all = nt + 32 * kRgServe;
-  // the scale of m's digits: one place above the last vector's maximum (over
-  // an iteration m's grows by at most 1.3 and shrinks to no less than 0.3 on
+  // the scale of m's digits (of its entries times their columns' powers of two):
+  // one place above the last vector's maximum (over an iteration m's grows by at most 1.3 and shrinks to no less than 0.3 on
   // these systems); for the first m, which is like M^-1 A u, u's
   auto next_scale = [](int emax) { return emax < kFxExpMin || emax > kFxExpMax ? kFxNone : emax - 1022 + 1; };
   int E = next_scale(sh.emax);
@@ -539,7 +542,7 @@ __device__ __forceinline__ void resident_body(const ResidentArgs& P, unsigned ch
       bar_arrive(kBarDots, nt + 96);
       const double m = precond(wv);
       if (valid) {
-        const int2 d = fx_digits(m, E);
+        const int2 d = fx_digits(m, E - kc);
         if constexpr (CL) {
           *reinterpret_cast<int2*>(mdig + par * mrow + m_own) = d;
           *reinterpret_cast<double*>(mdig + (2 + par) * mrow + m_own) = m;
@@ -548,7 +551,7 @@ __device__ __forceinline__ void resident_body(const ResidentArgs& P, unsigned ch
           P.m[par][i] = m;
         }
       }
-      const int e = __reduce_max_sync(0xffffffffu, valid ? fx_biased_exp(m) : 0);
+      const int e = __reduce_max_sync(0xffffffffu, valid ? fx_biased_exp(m, kc) : 0);
       if (lane == 0) sh.ew[w] = e;
       __syncwarp();
       bar_arrive(kBarM, nt + 32);
@@ -562,7 +565,7 @@ __device__ __forceinline__ void resident_body(const ResidentArgs& P, unsigned ch
       bar_sync(kBarStep, all);
       stamp(3);
       if (sh.stop[par]) break;
-      const int top = sh.emax - 1022;          // 2^top is above m
+      const int top = sh.emax - 1022;          // 2^top is above m's scaled entries
       if (valid && (top > E || top < E - kFxSlack || !row_fx))
         n = row_product_m<CL>(P.A + 9 * (size_t)kb, cols, ke - kb, t10, rsub, P.m[par], (2 + par) * mrow);
       E = next_scale(sh.emax);
@@ -863,6 +866,7 @@ od_status resident_solve(Scene* s, const double* d_b, double* d_x, int pkind, do
   a.warps = R.warps;
   a.rp = s->bsr.row_ptr;
   a.col = s->bsr.col;
+  a.diag = s->bsr.diag_pos;
   a.A = s->A64;
   a.b = d_b;
   a.x = d_x;

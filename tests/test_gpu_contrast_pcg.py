@@ -1,0 +1,69 @@
+"""FP64 PCG on matrices of two materials (mass + h^2 K, a stiff half at the fixed end and a soft one, or stiff elements
+strewn in soft ones), as a host program that keeps its own element values hands them over: solves meet the tolerance they
+are asked for, in the iterations that the same preconditioner takes in the oracle.
+
+Bounds: a solve's true residual is verified to the tolerance (1 + 1e-6); the oracle's product that checks it carries its own
+rounding, 40 2^-53 |A| |x| (rows of some 40 entries).  Iterations as the other PCG tests hold them (the larger of 2 and
+3%); with strewn stiffness 6%: the pipelined recurrence's rounding costs it some of the last digits (60-bit digits and FP64
+products, emulated: 361 against 351 of the two-term recurrence at 1e-8, 440 against 437)."""
+import functools
+
+import numpy as np
+import pytest
+
+from opendeformer_gb300 import api, meshgen
+from oracle import restated
+from tests.gpu_util import ctx
+
+pytestmark = pytest.mark.gpu
+
+# free block rows: 128 (a cluster), 2,400 (the grid)
+SMALL, LARGE = (8, 3, 3), (24, 9, 9)
+
+
+@functools.lru_cache(maxsize=None)
+def system(dims, contrast, layout="half"):
+    g = meshgen.tet_grid(*dims, h=0.05, jitter=0.15, seed=1)
+    cd = meshgen.constrained_dofs_for_nodes(g.face_nodes(0, 0))
+    o = restated.OracleScene(g.X, g.tets, g.facets, cd, "corotational", 1000.0, 98640.0, 0.4506, 0.1)
+    x = g.X[g.tets].mean(axis=1)[:, 0] / g.X[:, 0].max()
+    if layout == "graded":
+        factor = contrast ** x
+    else:
+        stiff = x < 0.5 if layout == "half" else np.random.default_rng(6).random(len(x)) < 0.3
+        factor = np.where(stiff, contrast, 1.0)
+    emap = o.pattern()[3]
+    K = np.zeros(o.n_values)
+    np.add.at(K, emap[emap >= 0], (o.element_values()[0] * factor[:, None])[emap >= 0])
+    if contrast == 1:
+        assert np.abs(K - o.assemble()[0]).max() <= 1e-13 * np.abs(K).max()
+    return g, cd, o, K / 240.0 ** 2 + o.mass(), np.random.default_rng(2).normal(size=o.dofs)
+
+
+def solve(dims, contrast, layout, tol, precond, share, start=False):
+    g, cd, o, A, b = system(dims, contrast, layout)
+    s = api.Scene(ctx(), g.X, g.tets, g.facets, cd, api.CorotationalHyperelasticMaterial(1000.0, 98640.0, 0.4506, 0.1))
+    x0 = np.random.default_rng(3).normal(size=o.dofs) if start else None
+    x, st = s.pcg(A, b, x0, api.CGSolver(tol, 5000, api.Preconditioner(precond)))
+    s.close()
+    assert st.status == 0
+    true = np.linalg.norm(b - o.spmdv(A, x)) / np.linalg.norm(b)
+    rounding = 40 * 2.0 ** -53 * np.linalg.norm(o.spmdv(np.abs(A), np.abs(x))) / np.linalg.norm(b)
+    assert true <= tol * (1 + 1e-6) + rounding
+    assert abs(true - st.rel_residual) <= 2 * rounding
+    if share:
+        _, its = o.pcg(A, b, x0, tol=tol, maxit=5000, precond=precond)
+        assert abs(st.iterations - its) <= max(2, share * its)
+
+
+@pytest.mark.parametrize("contrast", [1, 1e4, 1e6, 1e7, 1e8])
+@pytest.mark.parametrize("tol", [1e-8, 1e-10])
+@pytest.mark.parametrize("dims,precond", [(SMALL, "jacobi"), (SMALL, "block_jacobi"), (LARGE, "block_jacobi")])
+def test_two_materials(dims, precond, tol, contrast):
+    solve(dims, contrast, "half", tol, precond, 0.03)
+
+
+@pytest.mark.parametrize("contrast", [1e4, 1e6, 1e8])
+@pytest.mark.parametrize("precond", ["jacobi", "block_jacobi"])
+def test_strewn_stiffness(precond, contrast):
+    solve(SMALL, contrast, "strewn", 1e-8, precond, 0.06)
