@@ -109,7 +109,8 @@ typedef struct od_solver_params {
 } od_solver_params;
 
 typedef struct od_solve_stats {
-  int iterations;       /* total inner iterations */
+  int iterations;       /* total inner iterations (a chip-resident FP64 solve that is started again in
+                           another recurrence: those of the one that x is from) */
   int refinements;      /* mixed: outer sweeps */
   double rel_residual;  /* ||b - A x|| / ||b|| at exit (FP64) */
   double ic_shift;      /* IC(0) diagonal shift used */

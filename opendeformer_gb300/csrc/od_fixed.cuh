@@ -36,9 +36,9 @@ __device__ __forceinline__ int fx_biased_exp(double v) { return (__double2hiint(
 // 2.7e-5; with k_c it follows FP64's (up to 1e8, none / Jacobi / block-Jacobi,
 // 60-bit digits emulated on the CPU).  Half the exponent does too down to 1e-8,
 // and ends at 1.5e-10 for 1e-10 at 1e8.
+constexpr int kFxColumnExp = 400;   // most of it, so that zeros stay below kFxExpMin and NaN above kFxExpMax
 __device__ __forceinline__ int fx_column_exp(double diag) {
-  const int e = fx_biased_exp(diag);
-  return e == 0 || e == 0x7ff ? 0 : e - 1023;
+  return min(max(fx_biased_exp(diag) - 1023, -kFxColumnExp), kFxColumnExp);
 }
 // v 2^k, on the integer units; zero below the normal range (subnormal v too), infinite above it
 __device__ __forceinline__ double fx_times_pow2(double v, int k) {
@@ -48,11 +48,8 @@ __device__ __forceinline__ double fx_times_pow2(double v, int k) {
   if (e + k >= 0x7ff) return __hiloint2double((hi & (int)0x80000000) | 0x7ff00000, 0);
   return __hiloint2double(hi + k * (1 << 20), __double2loint(v));
 }
-// the biased exponent of v 2^k: 0 for zero, far beyond kFxExpMax for infinities and NaN
-__device__ __forceinline__ int fx_biased_exp(double v, int k) {
-  const int e = fx_biased_exp(v);
-  return e == 0 ? 0 : e == 0x7ff ? 8191 : max(e + k, 0);
-}
+// the biased exponent of v 2^k, k a column's: outside kFxExpMin .. kFxExpMax for zero, infinities and NaN
+__device__ __forceinline__ int fx_biased_exp(double v, int k) { return fx_biased_exp(v) + k; }
 
 // digits of v at the scale E; a magnitude of 2^E and more is cut off (the
 // caller's check has failed then), subnormal numbers are zero

@@ -49,6 +49,7 @@ struct SolveScalars {           // device-resident PCG scalars
   double rz[2];                 // r.z by iteration parity
   double rr, bb, eps, rr0, tr_num, tr_den, alpha, beta;
   int iter, max_iter, done, status;
+  int best;                     // chip-resident form: the iteration of the smallest r.r
 };
 
 struct SliceSys;
@@ -619,8 +620,9 @@ od_status mixed_ic0_solve(Scene* s, const double* d_b, double* d_x, const od_sol
 // PCG on A64; b and x are device vectors of length n_pad
 od_status resident_plan(Scene* s);
 void resident_free(ResidentPlan* R);
-od_status resident_solve(Scene* s, const double* d_b, double* d_x, int pkind, double tol, int max_iter, bool x_zero,
-                         unsigned long long* prof);
+// patience: iterations without a smaller residual after which it gives up (OD_ERR_NOT_CONVERGED), 0: none
+od_status resident_solve(Scene* s, const double* d_b, double* d_x, int pkind, double tol, int max_iter, int patience,
+                         bool x_zero, unsigned long long* prof);
 // the one-launch fixed-point PCG of systems beyond the resident one (od_wide.cu)
 od_status wide_build(Scene* s, WidePlan** out);
 od_status wide_solve(Scene* s, WidePlan* W, const double* d_b, double* d_x, int pkind, double tol, int max_iter, bool x_zero,

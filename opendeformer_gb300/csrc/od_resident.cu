@@ -82,7 +82,7 @@ struct ResidentArgs {
   double* m[2];                 // M^-1 w by iteration parity (not the cluster form)
   int2* mx[2];                  // its digits
   const double* pinv;
-  int pkind, x_zero, max_iter;
+  int pkind, x_zero, max_iter, patience;
   double tol;
   double* part;                 // 2 x 3 x gridDim.x partial sums
   int* epart;                   // 2 x gridDim.x largest exponents
@@ -121,7 +121,7 @@ struct ResidentShared {
   // first sum warp may be writing the next round's.  That one's next write of
   // the same word lies behind a kBarStep that the sync warp takes part in
   int stop[2];
-  int status, iter;
+  int status, iter, best, stalled;
   int emax;                     // the last vector's largest biased exponent
   int ew[kRgMaxWarps];          // its worker warps'
   int fail;                     // a wait ran out
@@ -307,25 +307,46 @@ template <bool CL>
 __device__ __noinline__ int stage_rows(const ResidentArgs& P, double* raw, unsigned* cols, unsigned mx, int steps, int kb,
                                        int ke, int row, int t, int r) {
   int em = 0;
-#pragma unroll 4
-  for (int j = 0; j < steps; j++) {
-    const bool in = kb + j < ke;
-    const double* a = P.A + 9 * (size_t)(kb + j) + 3 * r;
-    const int cb = in ? P.col[kb + j] : min(row, P.nb - 1);
-    const double* d = P.A + 9 * (size_t)P.diag[cb];
+  constexpr int kAhead = 16;   // columns whose diagonal blocks are looked up together: two round trips for all
+#pragma unroll 1
+  for (int j0 = 0; j0 < steps; j0 += kAhead) {
+    int dp[kAhead];
 #pragma unroll
-    for (int c = 0; c < 3; c++) {
-      const double v = in ? fx_times_pow2(a[c], -fx_column_exp(d[4 * c])) : 0.0;
-      raw[rg_value(j, r, 3 * t + c)] = v;
-      em = max(em, fx_biased_exp(v));
-    }
-    if (r == 0) {
-      unsigned at = kRgRowBytes * cb;
-      if constexpr (CL) {
-        const int g = cb / kRgRows, G = gridDim.x, c = ((g + 1) * G - 1) / P.ngroups;
-        at = cluster_addr(mx, c) + kRgRowBytes * (cb - kRgRows * (c * P.ngroups / G));
+    for (int u = 0; u < kAhead; u++) dp[u] = kb + j0 + u < ke ? P.col[kb + j0 + u] : min(row, P.nb - 1);
+#pragma unroll
+    for (int u = 0; u < kAhead; u++) {
+      if (r == 0 && j0 + u < steps) {
+        unsigned at = kRgRowBytes * dp[u];
+        if constexpr (CL) {
+          const int g = dp[u] / kRgRows, G = gridDim.x, c = ((g + 1) * G - 1) / P.ngroups;
+          at = cluster_addr(mx, c) + kRgRowBytes * (dp[u] - kRgRows * (c * P.ngroups / G));
+        }
+        cols[rg_column(j0 + u, t)] = at;
       }
-      cols[rg_column(j, t)] = at;
+      dp[u] = P.diag[dp[u]];
+    }
+#pragma unroll
+    for (int q = 0; q < kAhead; q += 4) {   // steps come in fours
+      if (j0 + q >= steps) break;
+      double v[4][3], d[4][3];
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const int k = kb + j0 + q + u;
+        const double *a = P.A + 9 * (size_t)k + 3 * r, *ad = P.A + 9 * (size_t)dp[q + u];
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+          v[u][c] = k < ke ? a[c] : 0.0;
+          d[u][c] = ad[4 * c];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+          const double x = fx_times_pow2(v[u][c], -fx_column_exp(d[u][c]));
+          raw[rg_value(j0 + q + u, r, 3 * t + c)] = x;
+          em = max(em, fx_biased_exp(x));
+        }
     }
   }
   unsigned long long sum = 0;
@@ -599,6 +620,9 @@ __device__ __forceinline__ void resident_body(const ResidentArgs& P, unsigned ch
     // sum warp j takes dot product j; the first forms the step lengths
     const int j = w - W - 1;
     double gam_inv = 0.0, den_k = 0.0;   // 1 / gamma and den / gamma^2 of the last iteration
+    // the third keeps count of the iterations without a smaller r.r (the first is
+    // what a round waits for): the iteration of the smallest, and its upper half
+    int best = 0, best_hi = 0x7fffffff;
 #pragma unroll 1
     for (int it = 0;; it++) {
       bar_sync(kBarDots, nt + 96);
@@ -609,7 +633,16 @@ __device__ __forceinline__ void resident_body(const ResidentArgs& P, unsigned ch
       __syncwarp();
       if (j > 0) {
         bar_arrive(kBarTot, 96);
+        if (__double2hiint(t) < best_hi) {
+          best_hi = __double2hiint(t);
+          best = it;
+        }
         bar_sync(kBarStep, all);
+        if (j == 2 && lane == 0) {   // read behind the next kBarTot
+          sh.best = best;
+          sh.stalled = P.patience > 0 && it + 1 - best > P.patience + (best >> 2);
+        }
+        __syncwarp();
         if (sh.stop[it & 1]) break;
         continue;
       }
@@ -627,6 +660,9 @@ __device__ __forceinline__ void resident_body(const ResidentArgs& P, unsigned ch
         status = OD_ERR_NAN;
       } else if (!(rr > eps) || it >= P.max_iter) {
         stop = 1;
+      } else if (sh.stalled) {
+        stop = 1;
+        status = OD_ERR_NOT_CONVERGED;
       } else if (!isfinite(alpha) || !isfinite(beta)) {
         stop = 1;
         status = OD_ERR_NAN;
@@ -674,6 +710,7 @@ __device__ __forceinline__ void resident_body(const ResidentArgs& P, unsigned ch
     sc->iter = sh.iter;
     sc->max_iter = P.max_iter;
     sc->status = sh.status;
+    sc->best = sh.best;
     sc->tr_num = sh.tot[0];
     sc->tr_den = bb;
     sc->done = 1;
@@ -686,7 +723,7 @@ __global__ void __launch_bounds__(32 * (MAXW + kRgServe), 1) pcg_resident_kernel
   __shared__ ResidentShared sh;
   if (threadIdx.x == 0) {
     sh.fail = 0;
-    sh.stop[0] = sh.stop[1] = 0;
+    sh.stop[0] = sh.stop[1] = sh.stalled = 0;
     sh.status = OD_OK;
     for (int k = 0; k < kPcgProfSlots; k++) sh.prof[k] = 0;
     if constexpr (CL)
@@ -840,8 +877,8 @@ void resident_free(ResidentPlan* R) {
   *R = ResidentPlan();
 }
 
-od_status resident_solve(Scene* s, const double* d_b, double* d_x, int pkind, double tol, int max_iter, bool x_zero,
-                         unsigned long long* prof) {
+od_status resident_solve(Scene* s, const double* d_b, double* d_x, int pkind, double tol, int max_iter, int patience,
+                         bool x_zero, unsigned long long* prof) {
   Pcg& P = s->pcg;
   ResidentPlan& R = P.res;
   if (!R.smem && !R.ell) {   // kept with the scene from its first such solve on
@@ -877,6 +914,7 @@ od_status resident_solve(Scene* s, const double* d_b, double* d_x, int pkind, do
   a.pkind = pkind;
   a.x_zero = x_zero;
   a.max_iter = max_iter;
+  a.patience = patience;
   a.tol = tol;
   a.part = P.partial;
   a.epart = (int*)(P.partial + 6 * (size_t)R.grid);   // partial holds 8 per SM

@@ -3455,35 +3455,56 @@ od_status pcg_solve(Scene* s, const double* d_b, double* d_x, const od_solver_pa
       if (prof) OD_CUDA(cudaEventRecord(s->ctx->ev_pool[1], strm));
       return pcg_finish(s, d_b, d_x, shift, st, true, prof, phases);
     }
-    // chip-resident systems: the pipelined form of od_resident.cu.  Below 1e-9
-    // with its true residual verified, from the sizes on at which going on from
-    // the true residual takes at most about 1% more iterations (solves that run to
-    // their dimension part from it: preconditioned 1.5% at 105 DOFs, 0.7% at 252,
-    // 0.1% at 1,260; without a preconditioner 2.7% at 252, 1.1% at 720, 0.4% at
-    // 1,260, none at 12,000).  A call of 200 iterations at 1e-10: 252 DOFs 1,950
-    // -> 480 us, 1,260 2,500 -> 680, 4,860 2,760 -> 1,040; 260 iterations without a
-    // preconditioner 720 DOFs 3,150 -> 760, 12,870 3,500 -> 1,570
-    const int verify_rows = pk == OD_PRECOND_NONE ? 240 : 80;
-    const bool verify = P.recur < 0 && recur == 1 && nb >= verify_rows;
-    if (P.res.warps > 0 && (recur == 2 || verify)) {
-      OD_TRY(resident_solve(s, d_b, d_x, pk, prm->tol, prm->max_iter, x_zero, profp));
+    // chip-resident systems: the pipelined form of od_resident.cu; below 1e-9
+    // from the sizes on at which going on from the true residual takes at most
+    // about 1% more iterations (solves that run to their dimension part from it:
+    // preconditioned 1.5% at 105 DOFs, 0.7% at 252, 0.1% at 1,260; without a
+    // preconditioner 2.7% at 252, 1.1% at 720, 0.4% at 1,260, none at 12,000).  A
+    // call of 200 iterations at 1e-10: 252 DOFs 1,950 -> 480 us, 1,260 2,500 ->
+    // 680, 4,860 2,760 -> 1,040; 260 iterations without a preconditioner 720 DOFs
+    // 3,150 -> 760, 12,870 3,500 -> 1,570
+    const int small_rows = pk == OD_PRECOND_NONE ? 240 : 80;
+    if (P.res.warps > 0 && (recur == 2 || (P.recur < 0 && recur == 1 && nb >= small_rows))) {
+      // The pipelined recurrences lose more to rounding than the others: on
+      // ill-conditioned systems their residual parts from the true one or comes
+      // down no further.  So (unless the form is asked for by name) the true
+      // residual decides.  Above the tolerance, a pass goes on from it for up to
+      // 2% more iterations; a solve that this does not end, or that has not come
+      // down for 400 iterations and a quarter of those before, starts again in the
+      // recurrence form, from the vector it was given.  Stiffness graded over 1e4,
+      // block-Jacobi, 1e-10 (emulated): 218 iterations there, none here; strewn
+      // stiffness comes down in steps of up to 192 iterations.
+      const bool decides = P.recur < 0;
+      if (decides && !x_zero) OD_CUDA(cudaMemcpyAsync(P.r, d_x, sizeof(double) * (size_t)n, cudaMemcpyDeviceToDevice, strm));
+      OD_TRY(resident_solve(s, d_b, d_x, pk, prm->tol, prm->max_iter, decides ? 400 : 0, x_zero, profp));
       if (prof) OD_CUDA(cudaEventRecord(s->ctx->ev_pool[1], strm));
-      if (!verify) return pcg_finish(s, d_b, d_x, shift, st, true, prof, phases);
-      // on from the true residual while it is above the tolerance by more
-      // than its own rounding, a few times at most
-      constexpr int kCycles = 4;
+      if (!decides) return pcg_finish(s, d_b, d_x, shift, st, true, prof, phases);
       od_solve_stats ss{};
-      OD_TRY(pcg_finish(s, d_b, d_x, shift, &ss, true, prof, phases));
-      for (int c = 0; c < kCycles && ss.status == OD_OK && ss.rel_residual > prm->tol * (1.0 + 1e-6); c++) {
-        const int left = prm->max_iter - ss.iterations, used = ss.iterations;
-        if (left <= 0) break;
+      od_status e = pcg_finish(s, d_b, d_x, shift, &ss, true, prof, phases);
+      auto met = [&] { return ss.status == OD_OK && ss.rel_residual <= prm->tol * (1.0 + 1e-6); };
+      // out of iterations on its way down: no fault of the form
+      const SolveScalars& h = *P.sc_host;
+      bool done = e != OD_OK || met() ||
+                  (ss.status == OD_ERR_NOT_CONVERGED && h.iter >= h.max_iter && h.iter - h.best <= 128 && h.tr_num <= 4.0 * h.rr);
+      const int most = std::min(prm->max_iter, ss.iterations + std::max(2, ss.iterations / 50));
+      while (!done && ss.status == OD_OK && ss.iterations < most) {
+        const int used = ss.iterations;
         OD_CUDA(cudaMemsetAsync(P.gbar, 0, sizeof(GridBarrier), strm));
-        OD_TRY(resident_solve(s, d_b, d_x, pk, prm->tol, left, false, nullptr));
-        OD_TRY(pcg_finish(s, d_b, d_x, shift, &ss, true, false));
+        OD_TRY(resident_solve(s, d_b, d_x, pk, prm->tol, most - used, 0, false, nullptr));
+        e = pcg_finish(s, d_b, d_x, shift, &ss, true, false);
+        if (ss.iterations == 0) break;   // the residual's own rounding
         ss.iterations += used;
+        done = e != OD_OK || met();
       }
-      if (st) *st = ss;
-      return OD_OK;
+      if (done) {
+        if (st) *st = ss;
+        return e;
+      }
+      if (x_zero) OD_CUDA(cudaMemsetAsync(d_x, 0, sizeof(double) * (size_t)n, strm));
+      else OD_CUDA(cudaMemcpyAsync(d_x, P.r, sizeof(double) * (size_t)n, cudaMemcpyDeviceToDevice, strm));
+      OD_CUDA(cudaMemsetAsync(P.gbar, 0, sizeof(GridBarrier), strm));
+      recur = 1;
+      if (prof) OD_CUDA(cudaEventRecord(s->ctx->ev_pool[0], strm));
     }
     OD_KL(s);
     OD_CUDA(cudaLaunchCooperativeKernel(fn, dim3(G2), dim3(kPThreads), args, dyn, strm));

@@ -58,7 +58,8 @@ def solve(dims, contrast, layout, tol, precond, share, start=False):
 
 @pytest.mark.parametrize("contrast", [1, 1e4, 1e6, 1e7, 1e8])
 @pytest.mark.parametrize("tol", [1e-8, 1e-10])
-@pytest.mark.parametrize("dims,precond", [(SMALL, "jacobi"), (SMALL, "block_jacobi"), (LARGE, "block_jacobi")])
+@pytest.mark.parametrize("precond", ["jacobi", "block_jacobi"])
+@pytest.mark.parametrize("dims", [SMALL, LARGE])
 def test_two_materials(dims, precond, tol, contrast):
     solve(dims, contrast, "half", tol, precond, 0.03)
 
@@ -67,3 +68,35 @@ def test_two_materials(dims, precond, tol, contrast):
 @pytest.mark.parametrize("precond", ["jacobi", "block_jacobi"])
 def test_strewn_stiffness(precond, contrast):
     solve(SMALL, contrast, "strewn", 1e-8, precond, 0.06)
+
+
+# where the pipelined recurrence's residual parts from the true one, or comes down no further (60-bit digits or FP64
+# products alike, emulated): 218 iterations of the two-term recurrence for the graded stiffness, none of the other
+
+
+@pytest.mark.parametrize("tol", [1e-8, 1e-10])
+@pytest.mark.parametrize("start", [False, True])
+@pytest.mark.parametrize("dims", [SMALL, LARGE])
+def test_graded_stiffness(dims, start, tol):
+    solve(dims, 1e4, "graded", tol, "block_jacobi", 0.06, start)
+
+
+@pytest.mark.parametrize("contrast", [1e4, 1e6, 1e7])
+@pytest.mark.parametrize("precond", ["jacobi", "block_jacobi"])
+def test_strewn_stiffness_to_the_last_digits(precond, contrast):
+    solve(SMALL, contrast, "strewn", 1e-10, precond, 0.06)
+
+
+@pytest.mark.parametrize("tol", [1e-8, 1e-10])
+def test_no_preconditioner(tol):
+    solve((12, 5, 5), 300, "half", tol, "none", None)
+
+
+def test_limits_are_kept():
+    """Solves that run out of iterations on their way down say so with as many as they were given."""
+    g, cd, o, A, b = system(SMALL, 1e4, "half")
+    s = api.Scene(ctx(), g.X, g.tets, g.facets, cd, api.CorotationalHyperelasticMaterial(1000.0, 98640.0, 0.4506, 0.1))
+    for n in (1, 7, 60):
+        for tol in (1e-8, 1e-10):
+            _, st = s.pcg(A, b, None, api.CGSolver(tol, n, api.BlockJacobiPreconditioner()))
+            assert st.status == 3 and st.iterations == n
