@@ -76,7 +76,7 @@ struct WideArgs {
   unsigned char* rec;        // per record [2][row of the block][30 lanes] digits of two steps (lane 3 t + c: column c of the group's row t), [10] the four columns, as byte offsets in zd
   int* ea;                   // [group][30] scales; then the flag
   int2* zd;                  // digits of the gathered vector, by places
-  double* zg;                // the vector itself, where digits cannot be had
+  double* zg;                // the vector itself, where digits cannot be had; x at the start and the end
   double *xg, *pg, *zv, *inv;   // x, p, z; the preconditioner [3][entries]; by places
   double tol;
   double* part;              // [2][3][G] partial sums
@@ -281,21 +281,21 @@ __device__ __noinline__ bool wide_sums(const WideArgs& P, WideShared& sh, double
   return !sh.fail;
 }
 
-// one row of A v in FP64 (v by places), for vectors and rows without a scale
+// one row of A v in FP64 (v by places): products with x, vectors and rows without a scale
 __device__ __noinline__ double wide_row64(const WideArgs& P, int g, int t, int r) {
   const int row = P.perm[kWdRows * g + t];
   if (row < 0) return 0.0;
   const int kb = P.rp[row], n = P.rp[row + 1] - kb;
-  double y = 0.0;
-#pragma unroll 2
+  double y0 = 0.0, y1 = 0.0, y2 = 0.0;
+#pragma unroll 6
   for (int j = 0; j < n; j++) {
     const double* a = P.A + 9 * (size_t)(kb + j) + 3 * r;
     const double* v = P.zg + 3 * (size_t)P.slot[P.col[kb + j]];
-    y = fma(a[0], __ldcg(v), y);
-    y = fma(a[1], __ldcg(v + 1), y);
-    y = fma(a[2], __ldcg(v + 2), y);
+    y0 = fma(a[0], __ldcg(v), y0);
+    y1 = fma(a[1], __ldcg(v + 1), y1);
+    y2 = fma(a[2], __ldcg(v + 2), y2);
   }
-  return y;
+  return (y0 + y1) + y2;
 }
 
 enum { kWdIterate, kWdStart, kWdEnd };
@@ -478,33 +478,31 @@ __device__ __forceinline__ void wide_body(const WideArgs& P, WideShared& sh, dou
   };
   const bool any64 = P.ea[kWdLanes * P.ngroups] != 0;   // a row without a scale
   const bool block = P.pkind == OD_PRECOND_BLOCK_JACOBI, diag = P.pkind == OD_PRECOND_JACOBI;
-  int ex = 0;
   for (int i = threadIdx.x; i < own; i += kWdThreads) {
     const int d = dof(i);
     const double b = d >= 0 ? P.b[d] : 0.0, x = d >= 0 && !P.x_zero ? P.x[d] : 0.0;
     X[i] = x;
     R[i] = b;
-    Z[i] = x;
     D[i] = Q[i] = 0.0;
-    ex = max(ex, fx_biased_exp(x));
+    if (!P.x_zero) __stcg(P.zg + kWdLanes * (size_t)c0 + i, x);
   }
   __syncthreads();
   unsigned es = 0;   // syncs so far
-  // a vector's digits (or the vector itself) for the next product; its largest
-  // exponent e is known to every CTA.  True: as digits
+  // z's digits (or z itself) for the next product; its largest exponent e is
+  // known to every CTA.  True: as digits
   int E = 0;
-  auto publish = [&](const double* v, int e) {
+  auto publish = [&](int e) {
     E = e - 1022;
     const bool fx = !any64 && e >= kFxExpMin && e <= kFxExpMax;
     for (int i = threadIdx.x; i < own; i += kWdThreads) {
-      if (fx) P.zd[kWdLanes * (size_t)c0 + i] = fx_digits(v[i], E);
-      else __stcg(P.zg + kWdLanes * (size_t)c0 + i, v[i]);
+      if (fx) P.zd[kWdLanes * (size_t)c0 + i] = fx_digits(Z[i], E);
+      else __stcg(P.zg + kWdLanes * (size_t)c0 + i, Z[i]);
     }
     return fx;
   };
   // z = M^-1 r, r.z and r.r of this thread's entries; digits: z's at the scale E
-  // too.  Only where a sync lies behind the last product: other CTAs may still be
-  // gathering what P.zd holds (at the start x's digits)
+  // too (not at the start, which has no scale yet).  A sync lies between the last
+  // product, whose gathers read what P.zd holds, and this
   double rz = 0.0, rr = 0.0;
   int ez = 0;
   auto precondition = [&](bool digits) {
@@ -537,12 +535,10 @@ __device__ __forceinline__ void wide_body(const WideArgs& P, WideShared& sh, dou
     t_prev = now;
   };
 
-  // ---- r = b - A x, z = M^-1 r
+  // ---- r = b - A x (products with x in FP64), z = M^-1 r
   if (!P.x_zero) {
-    if (!wide_sums<1>(P, sh, 0.0, 0.0, 0.0, ex, ++es)) return;
-    const bool fx = publish(X, sh.emax);
     if (!wide_sums<1>(P, sh, 0.0, 0.0, 0.0, 0, ++es)) return;
-    wide_product(P, sh, wd_dsm, kWdStart, 0.0, 0.0, fx, E);
+    wide_product(P, sh, wd_dsm, kWdStart, 0.0, 0.0, false, 0);
     __syncthreads();
   }
   double bb = 0.0;
@@ -567,7 +563,7 @@ __device__ __forceinline__ void wide_body(const WideArgs& P, WideShared& sh, dou
     const int e = sh.emax;
     bool fx = true;
     if (!ready || any64 || e < kFxExpMin || e > kFxExpMax || e - 1022 > E || E - (e - 1022) > kFxSlack) {
-      fx = publish(Z, e);
+      fx = publish(e);
       if (!wide_sums<1>(P, sh, 0.0, 0.0, 0.0, e, ++es)) return;
     }
     const double pq = wide_product(P, sh, wd_dsm, kWdIterate, alpha, beta, fx, E);
@@ -591,19 +587,16 @@ __device__ __forceinline__ void wide_body(const WideArgs& P, WideShared& sh, dou
     if (!isfinite(rr_now) || !isfinite(beta)) status = OD_ERR_NAN;
   }
 
-  // ---- the last x += alpha p, and the true residual ||b - A x||^2
-  ex = 0;
+  // ---- the last x += alpha p, and the true residual ||b - A x||^2, in FP64
   for (int i = threadIdx.x; i < own; i += kWdThreads) {
     const int d = dof(i);
     const double x = fma(alpha, D[i], X[i]);
     X[i] = x;
     if (d >= 0) P.x[d] = x;
-    ex = max(ex, fx_biased_exp(x));
+    __stcg(P.zg + kWdLanes * (size_t)c0 + i, x);
   }
-  if (!wide_sums<1>(P, sh, 0.0, 0.0, 0.0, ex, ++es)) return;
-  const bool fx = publish(X, sh.emax);
   if (!wide_sums<1>(P, sh, 0.0, 0.0, 0.0, 0, ++es)) return;
-  const double d2 = wide_product(P, sh, wd_dsm, kWdEnd, 0.0, 0.0, fx, E);
+  const double d2 = wide_product(P, sh, wd_dsm, kWdEnd, 0.0, 0.0, false, 0);
   if (!wide_sums<1>(P, sh, d2, 0.0, 0.0, 0, ++es)) return;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     SolveScalars* sc = P.sc;

@@ -100,3 +100,18 @@ def test_limits_are_kept():
         for tol in (1e-8, 1e-10):
             _, st = s.pcg(A, b, None, api.CGSolver(tol, n, api.BlockJacobiPreconditioner()))
             assert st.status == 3 and st.iterations == n
+
+
+@pytest.mark.parametrize("start", [False, True])
+@pytest.mark.parametrize("contrast", [1e6, 1e8])
+@pytest.mark.parametrize("dims", [SMALL, LARGE])
+def test_the_residual_of_the_form_for_large_systems(dims, contrast, start, monkeypatch):
+    """od_wide.cu reports the residual of its x, not that of x's digits (which at these contrasts are 1e-11 and 1e-9 off)."""
+    monkeypatch.setenv("OD_GB300_PCG_FORM", "wide")
+    g, cd, o, A, b = system(dims, contrast)
+    s = api.Scene(ctx(), g.X, g.tets, g.facets, cd, api.CorotationalHyperelasticMaterial(1000.0, 98640.0, 0.4506, 0.1))
+    x0 = np.random.default_rng(3).normal(size=o.dofs) if start else None
+    x, st = s.pcg(A, b, x0, api.CGSolver(1e-8, 5000, api.BlockJacobiPreconditioner()))
+    true = np.linalg.norm(b - o.spmdv(A, x)) / np.linalg.norm(b)
+    rounding = 40 * 2.0 ** -53 * np.linalg.norm(o.spmdv(np.abs(A), np.abs(x))) / np.linalg.norm(b)
+    assert abs(true - st.rel_residual) <= 2 * rounding
