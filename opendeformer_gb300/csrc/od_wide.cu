@@ -58,6 +58,7 @@ struct WidePlan {
   const int *cg = nullptr, *goff = nullptr, *perm = nullptr, *slot = nullptr;
   unsigned char* rec = nullptr;
   int* ea = nullptr;         // row scales; one more: whether a row has none
+  int* kx = nullptr;         // columns' powers of two, by places
   int2* zd = nullptr;
   double *zg = nullptr, *xg = nullptr, *pg = nullptr, *zv = nullptr, *inv = nullptr;
   unsigned* ctr = nullptr;
@@ -75,6 +76,8 @@ struct WideArgs {
   double* x;
   unsigned char* rec;        // per record [2][row of the block][30 lanes] digits of two steps (lane 3 t + c: column c of the group's row t), [10] the four columns, as byte offsets in zd
   int* ea;                   // [group][30] scales; then the flag
+  const int* diag;           // every block row's diagonal block
+  int* kx;                   // every place's power of two (fx_column_exp)
   int2* zd;                  // digits of the gathered vector, by places
   double* zg;                // the vector itself, where digits cannot be had; x at the start and the end
   double *xg, *pg, *zv, *inv;   // x, p, z; the preconditioner [3][entries]; by places
@@ -100,7 +103,14 @@ struct WideShared {
   int c0, c1;                              // this CTA's groups
 };
 
-// The matrix as digits, a warp per group: the scale of every row's sum of
+__global__ void __launch_bounds__(256) wide_scale_kernel(const __grid_constant__ WideArgs P) {
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= kWdLanes * P.ngroups) return;
+  const int row = P.perm[i / 3];
+  P.kx[i] = row >= 0 ? fx_column_exp(P.A[9 * (size_t)P.diag[row] + 4 * (i % 3)]) : 0;
+}
+
+// The matrix as digits, columns over their powers of two, a warp per group: the scale of every row's sum of
 // magnitudes (from the leading 21 bits of each value, rounded up), then the
 // digits.  Reads the matrix twice and writes it once: memory-bound.
 __global__ void __launch_bounds__(256) wide_stage_kernel(const __grid_constant__ WideArgs P, int first) {
@@ -109,22 +119,50 @@ __global__ void __launch_bounds__(256) wide_stage_kernel(const __grid_constant__
   const int t = lane / 3, r = lane % 3, row = P.perm[kWdRows * g + t];
   const int p0 = P.goff[g], np = P.goff[g + 1] - p0;
   const int kb = row >= 0 ? P.rp[row] : 0, n = row >= 0 ? P.rp[row + 1] - kb : 0;
+  unsigned char* rec0 = P.rec + (size_t)p0 * kWdRec;
+  const int4* at = reinterpret_cast<const int4*>(rec0 + 16 * 6 * kWdLanes) + t;   // a record's columns, kWdRec apart
+  auto columns = [&](int p) { return at[(size_t)p * (kWdRec / 16)]; };
+  if (first) {
+    if (r == 0)
+#pragma unroll 2
+      for (int p = 0; p < np; p++) {
+        int c[kWdSteps];
+#pragma unroll
+        for (int q = 0; q < kWdSteps; q++) {
+          const int j = kWdSteps * p + q;
+          c[q] = 24 * (j < n ? P.slot[P.col[kb + j]] : kWdRows * g + t);
+        }
+        reinterpret_cast<int4*>(rec0 + (size_t)p * kWdRec + 16 * 6 * kWdLanes)[t] = make_int4(c[0], c[1], c[2], c[3]);
+      }
+    __syncwarp((1u << kWdLanes) - 1);
+  }
   int em = 0;
   unsigned long long sum = 0;
-#pragma unroll 4
-  for (int j = 0; j < n; j++) {
-    const double* a = P.A + 9 * (size_t)(kb + j) + 3 * r;
+#pragma unroll 1
+  for (int p = 0; p < np; p++) {
+    const int4 c4 = columns(p);
+    const int c[kWdSteps] = {c4.x / 8, c4.y / 8, c4.z / 8, c4.w / 8};
+    double v[kWdSteps][3];
+    int k[kWdSteps][3];
 #pragma unroll
-    for (int c = 0; c < 3; c++) {
-      const double v = a[c];
-      const int hi = __double2hiint(v), e = (hi >> 20) & 0x7ff;
-      if (e > em) {
-        sum = (sum >> min(e - em, 63)) + 1;
-        em = e;
+    for (int q = 0; q < kWdSteps; q++)
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        v[q][i] = kWdSteps * p + q < n ? P.A[9 * (size_t)(kb + kWdSteps * p + q) + 3 * r + i] : 0.0;
+        k[q][i] = P.kx[c[q] + i];
       }
-      const int d = em - e;
-      sum += (d < 31 ? ((unsigned)((hi & 0xfffff) | 0x100000) + 1u) >> d : 0u) + 1u;
-    }
+#pragma unroll
+    for (int q = 0; q < kWdSteps; q++)
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        const int hi = __double2hiint(v[q][i]), e = fx_biased_exp(v[q][i], -k[q][i]);
+        if (e > em) {
+          sum = (sum >> min(e - em, 63)) + 1;
+          em = e;
+        }
+        const int d = em - e;
+        sum += (d < 31 ? ((unsigned)((hi & 0xfffff) | 0x100000) + 1u) >> d : 0u) + 1u;
+      }
   }
   const bool fits = em >= kFxExpMin && em <= kFxExpMax;
   const int ea = fits ? (64 - __clzll((long long)sum)) + em - 1043 : kFxNone;
@@ -136,30 +174,22 @@ __global__ void __launch_bounds__(256) wide_stage_kernel(const __grid_constant__
     for (int c = 0; c < 3; c++) P.inv[(size_t)c * ne + ent] = row >= 0 ? P.pinv[9 * (size_t)row + 3 * r + c] : 0.0;
 #pragma unroll 1
   for (int p = 0; p < np; p++) {
-    unsigned char* rec = P.rec + (size_t)(p0 + p) * kWdRec;
+    int4* rec = reinterpret_cast<int4*>(rec0 + (size_t)p * kWdRec);
+    const int4 c4 = columns(p);
+    const int c[kWdSteps] = {c4.x / 8, c4.y / 8, c4.z / 8, c4.w / 8};
+    int2 d[kWdSteps][3];
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
-      int2 d[2][3];
+    for (int q = 0; q < kWdSteps; q++)
 #pragma unroll
-      for (int q = 0; q < 2; q++) {
-        const int j = kWdSteps * p + 2 * h + q;
-        const double* a = P.A + 9 * (size_t)(kb + j) + 3 * r;
-#pragma unroll
-        for (int c = 0; c < 3; c++) d[q][c] = fits && j < n ? fx_digits(a[c], ea) : make_int2(0, 0);
-      }
-#pragma unroll
-      for (int c = 0; c < 3; c++)
-        reinterpret_cast<int4*>(rec)[(3 * h + r) * kWdLanes + 3 * t + c] = make_int4(d[0][c].x, d[0][c].y, d[1][c].x, d[1][c].y);
-    }
-    if (first && r == 0) {
-      int at[kWdSteps];
-#pragma unroll
-      for (int q = 0; q < kWdSteps; q++) {
+      for (int i = 0; i < 3; i++) {
         const int j = kWdSteps * p + q;
-        at[q] = 24 * (j < n ? P.slot[P.col[kb + j]] : kWdRows * g + t);
+        d[q][i] = fits && j < n ? fx_digits(P.A[9 * (size_t)(kb + j) + 3 * r + i], ea + P.kx[c[q] + i]) : make_int2(0, 0);
       }
-      reinterpret_cast<int4*>(rec + 16 * 6 * kWdLanes)[t] = make_int4(at[0], at[1], at[2], at[3]);
-    }
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+#pragma unroll
+      for (int i = 0; i < 3; i++)
+        rec[(3 * h + r) * kWdLanes + 3 * t + i] = make_int4(d[2 * h][i].x, d[2 * h][i].y, d[2 * h + 1][i].x, d[2 * h + 1][i].y);
   }
 }
 
@@ -472,6 +502,7 @@ __device__ __forceinline__ void wide_body(const WideArgs& P, WideShared& sh, dou
          *Z = P.zv + kWdLanes * (size_t)c0;
   const size_t ne = kWdLanes * (size_t)P.ngroups;
   const double* I = P.inv + kWdLanes * (size_t)c0;
+  const int* KX = P.kx + kWdLanes * (size_t)c0;
   auto dof = [&](int i) {
     const int row = P.perm[kWdRows * c0 + i / 3];
     return row >= 0 ? 3 * row + i % 3 : -1;
@@ -495,7 +526,7 @@ __device__ __forceinline__ void wide_body(const WideArgs& P, WideShared& sh, dou
     E = e - 1022;
     const bool fx = !any64 && e >= kFxExpMin && e <= kFxExpMax;
     for (int i = threadIdx.x; i < own; i += kWdThreads) {
-      if (fx) P.zd[kWdLanes * (size_t)c0 + i] = fx_digits(Z[i], E);
+      if (fx) P.zd[kWdLanes * (size_t)c0 + i] = fx_digits(Z[i], E - KX[i]);
       else __stcg(P.zg + kWdLanes * (size_t)c0 + i, Z[i]);
     }
     return fx;
@@ -508,7 +539,9 @@ __device__ __forceinline__ void wide_body(const WideArgs& P, WideShared& sh, dou
   auto precondition = [&](bool digits) {
     rz = rr = 0.0;
     ez = 0;
+#pragma unroll 3
     for (int i = threadIdx.x; i < own; i += kWdThreads) {
+      const int k = KX[i];
       const double r = R[i];
       double z = r;
       if (block) {
@@ -518,8 +551,8 @@ __device__ __forceinline__ void wide_body(const WideArgs& P, WideShared& sh, dou
         z = I[i] * r;
       }
       Z[i] = z;
-      if (digits) P.zd[kWdLanes * (size_t)c0 + i] = fx_digits(z, E);
-      ez = max(ez, fx_biased_exp(z));
+      if (digits) P.zd[kWdLanes * (size_t)c0 + i] = fx_digits(z, E - k);
+      ez = max(ez, fx_biased_exp(z, k));
       rz = fma(r, z, rz);
       rr = fma(r, r, rr);
     }
@@ -661,6 +694,7 @@ void wide_free(WidePlan* W) {
   cudaFree(W->ints);
   cudaFree(W->rec);
   cudaFree(W->ea);
+  cudaFree(W->kx);
   cudaFree(W->zd);
   cudaFree(W->zg);
   cudaFree(W->xg);
@@ -746,6 +780,7 @@ od_status wide_build(Scene* s, WidePlan** out) {
   cudaError_t e = cudaMalloc(&W.ints, sizeof(int) * ints.size());
   if (e == cudaSuccess) e = cudaMalloc(&W.rec, b_rec);
   if (e == cudaSuccess) e = cudaMalloc(&W.ea, b_ea);
+  if (e == cudaSuccess) e = cudaMalloc(&W.kx, b_ea);
   if (e == cudaSuccess) e = cudaMalloc(&W.zd, b_vec);
   if (e == cudaSuccess) e = cudaMalloc(&W.zg, b_vec);
   if (e == cudaSuccess) e = cudaMalloc(&W.xg, b_vec);
@@ -763,7 +798,7 @@ od_status wide_build(Scene* s, WidePlan** out) {
   }
   for (int k = 0; k < 4; k++) *dst[k] = W.ints + offs[k];
   *made = W;
-  s->device_bytes += (long long)(sizeof(int) * ints.size() + b_rec + b_inv + b_ea + 5 * b_vec + b_ctr);
+  s->device_bytes += (long long)(sizeof(int) * ints.size() + b_rec + b_inv + 2 * b_ea + 5 * b_vec + b_ctr);
   *out = made;
   return OD_OK;
 }
@@ -793,6 +828,8 @@ od_status wide_solve(Scene* s, WidePlan* W, const double* d_b, double* d_x, int 
   a.x = d_x;
   a.rec = W->rec;
   a.ea = W->ea;
+  a.diag = s->bsr.diag_pos;
+  a.kx = W->kx;
   a.zd = W->zd;
   a.zg = W->zg;
   a.xg = W->xg;
@@ -808,6 +845,9 @@ od_status wide_solve(Scene* s, WidePlan* W, const double* d_b, double* d_x, int 
   a.prof = prof;
   OD_CUDA(cudaMemsetAsync(W->ctr, 0, sizeof(unsigned) * 4 * kWdCtr, st));
   OD_CUDA(cudaMemsetAsync(W->ea + kWdLanes * (size_t)W->ngroups, 0, sizeof(int), st));
+  OD_KL(s);
+  wide_scale_kernel<<<(kWdLanes * W->ngroups + 255) / 256, 256, 0, st>>>(a);
+  OD_CUDA(cudaGetLastError());
   OD_KL(s);
   wide_stage_kernel<<<(W->ngroups + 7) / 8, 256, 0, st>>>(a, W->staged ? 0 : 1);
   OD_CUDA(cudaGetLastError());
