@@ -338,10 +338,13 @@ __device__ void polar3(const FT* F, FT* R) {
   const FT inv3 = FT(0.333333333333333333333333);
   FT lam;
   if (b >= tau - inv3) {
-    // the closed form in FP32, then two Newton steps (the derivative's
-    // reciprocal need not be better than FP32) -- FP64 roots, quotients and
-    // transcendental functions are long sequences on the FP64 units; the
-    // closed form in FP64 where the root is close to another
+    // the closed form in FP32, then two steps with that start's derivative --
+    // FP64 roots, quotients and transcendental functions are long sequences on
+    // the FP64 units.  The start and the derivative are as far off as the root is
+    // close to another: two steps leave 1e-14 of the root's error at derivatives
+    // above 0.5, but 3e-13 at 0.1-0.2 and 6e-12 at 0.05 (flat and inverted
+    // elements), where a third leaves 1e-14 as well; the closed form in FP64
+    // leaves 2e-14 there, and is taken below
     const FT c = FT(8) * dA;
     const float cf = (float)c, bf = (float)b;
     const float d0 = 1.f + 3.f * bf, s0 = sqrtf(d0), al0 = (-1.f + (27.f / 16.f) * cf * cf + 9.f * bf) / (d0 * s0);
@@ -352,6 +355,7 @@ __device__ void polar3(const FT* F, FT* R) {
       lam = (FT)l0;
       lam -= (lam * (lam * (lam * lam - FT(2)) - c) + b) * rd;
       lam -= (lam * (lam * (lam * lam - FT(2)) - c) + b) * rd;
+      if (df < 0.5f) lam -= (lam * (lam * (lam * lam - FT(2)) - c) + b) * rd;
     } else {
       FT D0 = FT(1) + FT(3) * b;
       FT D1 = FT(-1) + (FT(27) / FT(16)) * c * c + FT(9) * b;
