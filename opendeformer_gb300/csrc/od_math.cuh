@@ -655,7 +655,8 @@ template <class FT>
 __device__ void psd3(FT* m) {
   // Positive leading minors (Sylvester) prove every eigenvalue positive, in
   // which case the projection leaves the matrix unchanged: skip the eigensolve.
-  // (in FP32 first: minors far enough above their rounding settle it)
+  // (in FP32 first: minors far enough above their rounding, and products far
+  // enough above the subnormal numbers, settle it)
   {
     float f[6];
 #pragma unroll
@@ -664,7 +665,9 @@ __device__ void psd3(FT* m) {
     const float m01 = f[0] * f[3] - f[1] * f[1], dt = f[0] * c0 - f[1] * c1 + f[2] * c2;
     const float big = fabsf(f[0]) * (fabsf(f[3] * f[5]) + f[4] * f[4]) + fabsf(f[1]) * (fabsf(f[1] * f[5]) + fabsf(f[4] * f[2])) +
                       fabsf(f[2]) * (fabsf(f[1] * f[4]) + fabsf(f[3] * f[2]));
-    if (f[0] > 0.f && m01 > 1e-5f * fabsf(f[0] * f[3]) && dt > 1e-5f * big && big < 1e37f) return;
+    if (f[0] > 0.f && m01 > 1e-5f * fabsf(f[0] * f[3]) && dt > 1e-5f * big && big < 1e37f && big > 1e-30f &&
+        f[0] * f[3] > 1e-30f && f[3] * f[5] > 1e-30f)
+      return;
   }
   {
     const FT m01 = m[0] * m[3] - m[1] * m[1];
