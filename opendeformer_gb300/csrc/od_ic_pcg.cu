@@ -666,7 +666,8 @@ static void ic_pcg_config(int grid, size_t smem, bool cluster, cudaStream_t st, 
 // The factor's structure from the colour order (order: the system's block row
 // of every factor row; cstart: first factor row of every colour).  *out stays
 // null when the launches do not take the system: too many colours, rows too
-// long, vectors or a row's blocks and pairs that do not fit shared memory.
+// long, vectors or a row's blocks and pairs that do not fit shared memory, no
+// device memory for it.
 od_status ic_pcg_build(Scene* s, const std::vector<int>& rp, const std::vector<int>& col, const std::vector<int>& order,
                        const std::vector<int>& cstart, IcPcg** out) {
   *out = nullptr;
@@ -872,10 +873,10 @@ od_status ic_pcg_build(Scene* s, const std::vector<int>& rp, const std::vector<i
   }
   const size_t nv = 2 * (size_t)kIpVals * ((size_t)nfs + nbs + nt) + (size_t)kIpVals * nfs + 2 * ((size_t)kIpEnts * nt + 1);
   const size_t nctr = 4 * kIpCtr + kIpShifts, nadr = I.cluster ? (size_t)kIpEnts * (nfs + nbs) : 0;
-  cudaError_t e = cudaMalloc(&I.ints, sizeof(int) * all.size());
-  if (e == cudaSuccess) e = cudaMalloc(&I.vals, sizeof(double) * nv);
-  if (e == cudaSuccess) e = cudaMalloc(&I.ctr, sizeof(unsigned) * nctr);
-  if (e == cudaSuccess && nadr) e = cudaMalloc(&I.adr, sizeof(unsigned) * nadr);
+  cudaError_t e = plan_malloc(&I.ints, sizeof(int) * all.size());
+  if (e == cudaSuccess) e = plan_malloc(&I.vals, sizeof(double) * nv);
+  if (e == cudaSuccess) e = plan_malloc(&I.ctr, sizeof(unsigned) * nctr);
+  if (e == cudaSuccess && nadr) e = plan_malloc(&I.adr, sizeof(unsigned) * nadr);
   if (e == cudaSuccess) e = cudaMemcpy(I.ints, all.data(), sizeof(int) * all.size(), cudaMemcpyHostToDevice);
   // places no block has are never written: zero
   if (e == cudaSuccess) e = cudaMemsetAsync(I.vals, 0, sizeof(double) * nv, s->ctx->stream);
@@ -884,7 +885,9 @@ od_status ic_pcg_build(Scene* s, const std::vector<int>& rp, const std::vector<i
     cudaFree(I.vals);
     cudaFree(I.ctr);
     cudaFree(I.adr);
-    return cuda_fail(e, "IC(0) structure");
+    if (e != cudaErrorMemoryAllocation) return cuda_fail(e, "IC(0) structure");
+    cudaGetLastError();   // no room for it: the separate launches need less
+    return OD_OK;
   }
   for (int k = 0; k < kArrays; k++) *dst[k] = I.ints + offs[k];
   s->device_bytes += (long long)(sizeof(int) * all.size() + sizeof(double) * nv + sizeof(unsigned) * (nctr + nadr));

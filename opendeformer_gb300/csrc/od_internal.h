@@ -618,6 +618,11 @@ od_status mixed_ic0_solve(Scene* s, const double* d_b, double* d_x, const od_sol
                           od_solve_stats* st);
 
 // PCG on A64; b and x are device vectors of length n_pad
+// device memory of a solver's plan, without which the solve takes a form that
+// needs less.  OD_GB300_PLAN_BYTES: the most that one such array may take
+cudaError_t plan_malloc_bytes(void** p, size_t bytes);
+template <class T>
+cudaError_t plan_malloc(T** p, size_t bytes) { return plan_malloc_bytes((void**)p, bytes); }
 od_status resident_plan(Scene* s);
 void resident_free(ResidentPlan* R);
 // patience: iterations without a smaller residual after which it gives up (OD_ERR_NOT_CONVERGED), 0: none

@@ -2619,6 +2619,12 @@ od_status ic0_check(Scene* s) {
   return OD_OK;
 }
 
+cudaError_t plan_malloc_bytes(void** p, size_t bytes) {
+  const char* most = std::getenv("OD_GB300_PLAN_BYTES");
+  if (most && bytes > std::strtoull(most, nullptr, 10)) return cudaErrorMemoryAllocation;
+  return cudaMalloc(p, bytes);
+}
+
 od_status pcg_alloc(Scene* s) {
   Pcg& P = s->pcg;
   const int n = 3 * s->bsr.nb;

@@ -777,17 +777,17 @@ od_status wide_build(Scene* s, WidePlan** out) {
   const size_t b_rec = (size_t)kWdRec * W.records, b_inv = 3 * sizeof(double) * kWdLanes * (size_t)W.ngroups,
                b_ea = sizeof(int) * (kWdLanes * (size_t)W.ngroups + 1), b_vec = sizeof(double) * kWdLanes * (size_t)W.ngroups,
                b_ctr = sizeof(unsigned) * 4 * kWdCtr + sizeof(double) * 6 * G + sizeof(int) * 2 * G;
-  cudaError_t e = cudaMalloc(&W.ints, sizeof(int) * ints.size());
-  if (e == cudaSuccess) e = cudaMalloc(&W.rec, b_rec);
-  if (e == cudaSuccess) e = cudaMalloc(&W.ea, b_ea);
-  if (e == cudaSuccess) e = cudaMalloc(&W.kx, b_ea);
-  if (e == cudaSuccess) e = cudaMalloc(&W.zd, b_vec);
-  if (e == cudaSuccess) e = cudaMalloc(&W.zg, b_vec);
-  if (e == cudaSuccess) e = cudaMalloc(&W.xg, b_vec);
-  if (e == cudaSuccess) e = cudaMalloc(&W.pg, b_vec);
-  if (e == cudaSuccess) e = cudaMalloc(&W.zv, b_vec);
-  if (e == cudaSuccess) e = cudaMalloc(&W.inv, b_inv);
-  if (e == cudaSuccess) e = cudaMalloc(&W.ctr, b_ctr);
+  cudaError_t e = plan_malloc(&W.ints, sizeof(int) * ints.size());
+  if (e == cudaSuccess) e = plan_malloc(&W.rec, b_rec);
+  if (e == cudaSuccess) e = plan_malloc(&W.ea, b_ea);
+  if (e == cudaSuccess) e = plan_malloc(&W.kx, b_ea);
+  if (e == cudaSuccess) e = plan_malloc(&W.zd, b_vec);
+  if (e == cudaSuccess) e = plan_malloc(&W.zg, b_vec);
+  if (e == cudaSuccess) e = plan_malloc(&W.xg, b_vec);
+  if (e == cudaSuccess) e = plan_malloc(&W.pg, b_vec);
+  if (e == cudaSuccess) e = plan_malloc(&W.zv, b_vec);
+  if (e == cudaSuccess) e = plan_malloc(&W.inv, b_inv);
+  if (e == cudaSuccess) e = plan_malloc(&W.ctr, b_ctr);
   if (e == cudaSuccess) e = cudaMemcpy(W.ints, ints.data(), sizeof(int) * ints.size(), cudaMemcpyHostToDevice);
   WidePlan* made = new WidePlan(W);
   if (e != cudaSuccess) {
