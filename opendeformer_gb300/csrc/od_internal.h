@@ -625,6 +625,7 @@ template <class T>
 cudaError_t plan_malloc(T** p, size_t bytes) { return plan_malloc_bytes((void**)p, bytes); }
 od_status resident_plan(Scene* s);
 void resident_free(ResidentPlan* R);
+od_status resident_ready(Scene* s);   // its device memory; called before resident_solve
 // patience: iterations without a smaller residual after which it gives up (OD_ERR_NOT_CONVERGED), 0: none
 od_status resident_solve(Scene* s, const double* d_b, double* d_x, int pkind, double tol, int max_iter, int patience,
                          bool x_zero, unsigned long long* prof);

@@ -877,26 +877,40 @@ void resident_free(ResidentPlan* R) {
   *R = ResidentPlan();
 }
 
+// The plan's device memory, with the scene from its first such solve on; without
+// room for it the plan is given up (warps 0) and the persistent kernel of
+// od_sparse.cu takes the system.
+od_status resident_ready(Scene* s) {
+  ResidentPlan& R = s->pcg.res;
+  const bool ell = !R.smem && !R.ell, grid = !R.cluster && !R.ctr;
+  if (R.warps == 0 || !(ell || grid)) return OD_OK;
+  const size_t b_off = sizeof(int) * R.off.size(), b_ell = ell ? (size_t)std::max(1, R.off.back()) * kRgStepBytes : 0,
+               b_mx = 2 * 3 * sizeof(int2) * (size_t)s->bsr.nb, b_ctr = 4 * kCtrStride * sizeof(unsigned);
+  cudaError_t e = cudaSuccess;
+  if (ell) {
+    e = plan_malloc(&R.ell_off, b_off);
+    if (e == cudaSuccess) e = plan_malloc(&R.ell, b_ell);
+    if (e == cudaSuccess) e = cudaMemcpy(R.ell_off, R.off.data(), b_off, cudaMemcpyHostToDevice);
+  }
+  if (e == cudaSuccess && grid) {
+    e = plan_malloc(&R.mx, b_mx);
+    if (e == cudaSuccess) e = plan_malloc(&R.ctr, b_ctr);
+  }
+  if (e != cudaSuccess) {
+    resident_free(&R);
+    if (e != cudaErrorMemoryAllocation) return cuda_fail(e, "chip-resident PCG plan");
+    cudaGetLastError();
+    return OD_OK;
+  }
+  s->device_bytes += (long long)((ell ? b_off + b_ell : 0) + (grid ? b_mx + b_ctr : 0));
+  return OD_OK;
+}
+
 od_status resident_solve(Scene* s, const double* d_b, double* d_x, int pkind, double tol, int max_iter, int patience,
                          bool x_zero, unsigned long long* prof) {
   Pcg& P = s->pcg;
   ResidentPlan& R = P.res;
-  if (!R.smem && !R.ell) {   // kept with the scene from its first such solve on
-    const size_t bytes = (size_t)std::max(1, R.off.back()) * kRgStepBytes;
-    OD_CUDA(cudaMalloc(&R.ell_off, sizeof(int) * R.off.size()));
-    OD_CUDA(cudaMemcpy(R.ell_off, R.off.data(), sizeof(int) * R.off.size(), cudaMemcpyHostToDevice));
-    OD_CUDA(cudaMalloc(&R.ell, bytes));
-    s->device_bytes += (long long)(bytes + sizeof(int) * R.off.size());
-  }
-  if (!R.cluster) {
-    if (!R.ctr) {
-      const size_t bytes = 2 * 3 * sizeof(int2) * (size_t)s->bsr.nb;
-      OD_CUDA(cudaMalloc(&R.mx, bytes));
-      OD_CUDA(cudaMalloc(&R.ctr, 4 * kCtrStride * sizeof(unsigned)));
-      s->device_bytes += (long long)bytes;
-    }
-    OD_CUDA(cudaMemsetAsync(R.ctr, 0, 4 * kCtrStride * sizeof(unsigned), s->ctx->stream));
-  }
+  if (!R.cluster) OD_CUDA(cudaMemsetAsync(R.ctr, 0, 4 * kCtrStride * sizeof(unsigned), s->ctx->stream));
   ResidentArgs a{};
   a.nb = s->bsr.nb;
   a.ngroups = (s->bsr.nb + kRgRows - 1) / kRgRows;

@@ -3470,7 +3470,9 @@ od_status pcg_solve(Scene* s, const double* d_b, double* d_x, const od_solver_pa
     // 680, 4,860 2,760 -> 1,040; 260 iterations without a preconditioner 720 DOFs
     // 3,150 -> 760, 12,870 3,500 -> 1,570
     const int small_rows = pk == OD_PRECOND_NONE ? 240 : 80;
-    if (P.res.warps > 0 && (recur == 2 || (P.recur < 0 && recur == 1 && nb >= small_rows))) {
+    const bool resident = recur == 2 || (P.recur < 0 && recur == 1 && nb >= small_rows);
+    if (resident) OD_TRY(resident_ready(s));
+    if (resident && P.res.warps > 0) {
       // The pipelined recurrences lose more to rounding than the others: on
       // ill-conditioned systems their residual parts from the true one or comes
       // down no further.  So (unless the form is asked for by name) the true

@@ -13,8 +13,8 @@ from tests.gpu_util import ctx
 pytestmark = pytest.mark.gpu
 
 
-def check(precond, tol, monkeypatch, env=()):
-    g = meshgen.tet_grid(20, 8, 8, h=0.05, jitter=0.15, seed=4)
+def check(precond, tol, monkeypatch, env=(), dims=(20, 8, 8)):
+    g = meshgen.tet_grid(*dims, h=0.05, jitter=0.15, seed=4)
     cd = meshgen.constrained_dofs_for_nodes(g.face_nodes(0, 0))
     o = restated.OracleScene(g.X, g.tets, g.facets, cd, "neohookean", 1000.0, 98640.0, 0.4506, 0.1)
     o.set_displacements(np.random.default_rng(1).normal(scale=2e-4, size=g.X.shape))
@@ -37,3 +37,9 @@ def test_ic0_without_its_structure(monkeypatch):
 
 def test_large_systems_without_digits(monkeypatch):
     check("block_jacobi", 1e-10, monkeypatch, [("OD_GB300_PCG_FORM", "wide")])
+
+
+@pytest.mark.parametrize("smem", ["0", "1"])
+def test_chip_resident_systems_without_their_digits(smem, monkeypatch):
+    """The grid form (2,400 block rows), its matrix in L2 or in shared memory."""
+    check("block_jacobi", 1e-8, monkeypatch, [("OD_GB300_PCG_SMEM", smem)], (24, 9, 9))
