@@ -534,9 +534,11 @@ od_status od_scene_evaluate(od_scene* scene, double* values, double* f_int) {
   Scene* s = &scene->s;
   OD_CUDA(cudaSetDevice(s->ctx->device));
   // where the device reaches the host's arrays the assembly writes them as it
-  // goes, instead of two copies after it
-  double* hk = s->gat_kptr && values && host_reached(s->ctx, values) ? values : nullptr;
-  double* hf = s->gat_kptr && f_int && host_reached(s->ctx, f_int) ? f_int : nullptr;
+  // goes, instead of two copies after it (of arrays that overlap the forces'
+  // copy, the last, is what stays)
+  const bool direct = s->gat_kptr && (!values || !f_int || values + s->nvals <= f_int || f_int + s->dofs <= values);
+  double* hk = direct && values && host_reached(s->ctx, values) ? values : nullptr;
+  double* hf = direct && f_int && host_reached(s->ctx, f_int) ? f_int : nullptr;
   OD_TRY(launch_eval(s, true, false, hk, hf));
   if (values && !hk) OD_CUDA(cudaMemcpyAsync(values, s->K, sizeof(double) * s->nvals, cudaMemcpyDeviceToHost, s->ctx->stream));
   if (f_int && !hf) OD_CUDA(cudaMemcpyAsync(f_int, s->fint, sizeof(double) * s->dofs, cudaMemcpyDeviceToHost, s->ctx->stream));
