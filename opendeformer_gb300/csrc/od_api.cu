@@ -539,7 +539,10 @@ od_status od_scene_evaluate(od_scene* scene, double* values, double* f_int) {
   const bool direct = s->gat_kptr && (!values || !f_int || values + s->nvals <= f_int || f_int + s->dofs <= values);
   double* hk = direct && values && host_reached(s->ctx, values) ? values : nullptr;
   double* hf = direct && f_int && host_reached(s->ctx, f_int) ? f_int : nullptr;
-  OD_TRY(launch_eval(s, true, false, hk, hf));
+  // OD_GB300_ELEMENT_DF=1: the elements as mixed-precision solves evaluate them (to
+  // compare them with the FP64 ones)
+  const char* dfe = std::getenv("OD_GB300_ELEMENT_DF");
+  OD_TRY(launch_eval(s, true, dfe && dfe[0] == '1', hk, hf));
   if (values && !hk) OD_CUDA(cudaMemcpyAsync(values, s->K, sizeof(double) * s->nvals, cudaMemcpyDeviceToHost, s->ctx->stream));
   if (f_int && !hf) OD_CUDA(cudaMemcpyAsync(f_int, s->fint, sizeof(double) * s->dofs, cudaMemcpyDeviceToHost, s->ctx->stream));
   OD_TRY(sync_stream(s));

@@ -511,7 +511,8 @@ void ric_factor(const RicColumns& A, const double* values, double eps, double re
 constexpr int kElThreads = 64;
 od_status launch_precompute(Scene* s);
 od_status launch_mass(Scene* s);
-// K, fint at current u; with host_k and host_f (scenes with gather lists only,
+// K, fint at current u; refine: as the mixed-precision solves' elements (flat
+// ones by reciprocal roots, od_math.cuh); with host_k and host_f (scenes with gather lists only,
 // memory the device reaches) the assembly also writes them there: see od_api.cu
 od_status launch_eval(Scene* s, bool zero_first, bool refine, double* host_k = nullptr, double* host_f = nullptr);
 int element_precomputes();   // doubles per element in Scene::pre
