@@ -804,9 +804,9 @@ od_status ic_pcg_build(Scene* s, const std::vector<int>& rp, const std::vector<i
   I.factor_smem = (I.factor_warps * per_warp + 7) / 8 * 8;
   I.factor_grid = std::min(sms, kIpRows * nt);
   // One cluster while its 16 CTAs' FP64 units keep up with its barriers:
-  // measured 2.28 against the grid's 2.41 ms a step at 864 tasks (7,776 DOFs),
-  // 4.50 against 2.70 at 2,253 (OD_GB300_IC0_PCG=cluster, =grid: either form
-  // at any size).
+  // measured 2.24 against the grid's 2.38 ms a step at 864 tasks (7,776 DOFs),
+  // 2.36 against 2.32 at 972, 2.47 against 2.24 at 1,080, 4.29 against 2.59 at
+  // 2,253 (OD_GB300_IC0_PCG=cluster, =grid: either form at any size).
   constexpr int kClusterTasks = 896;
   const char* form = std::getenv("OD_GB300_IC0_PCG");
   const bool want_cluster = form ? form[0] == 'c' : nt <= kClusterTasks;

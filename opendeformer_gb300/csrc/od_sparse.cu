@@ -136,6 +136,9 @@ __device__ __forceinline__ double lower_row(int kb, int ke, int r, const int* __
   return acc;
 }
 
+// y (+)= c1 V1 x1 + c2 V2 x2 + c3 V3 x3 with V* read from the lower layout
+// through the full-BSR descriptors (SpMDV semantics, numerMethod.h:134-262).
+// Three lanes per block row as in the full-BSR product.
 template <int NSRC>
 __global__ void spmv_lower_kernel(int nb, const int* __restrict__ rp, const int* __restrict__ col,
                                   const int* __restrict__ kind, const int* __restrict__ off,
@@ -3441,8 +3444,11 @@ od_status pcg_solve(Scene* s, const double* d_b, double* d_x, const od_solver_pa
                              : (need <= 2 && prm->tol >= 1e-9 ? 2 : (prm->tol >= 1e-10 ? 1 : 0));
     if (recur == 2 && need > 2) recur = 1;
     // products in fixed point once the vectors are too long for two groups a
-    // warp: an iteration of 237,600 DOFs takes 32 us there and 43 here; at
-    // 161,568 (two groups) 25.4 and 26.7, and a solve's start takes 95 us more
+    // warp: an iteration of 237,600 DOFs takes 30.5 us there and 42.5 here.  At two
+    // groups the solve's start and end take 80-110 us more there, an iteration
+    // 21.9 us both at 95,040 DOFs, 22.7 against 28.7 at 126,720 and 25.4 against
+    // 30.2 at 161,568: solves of 72-90 iterations are 4% longer at the first and
+    // 10-18% shorter at the others
     const bool wide = P.recur < 0 ? recur == 1 && need > 2 : P.recur == 3;
     if (recur == 3) recur = 1;
     args[18] = (void*)&recur;
