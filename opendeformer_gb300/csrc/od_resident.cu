@@ -121,7 +121,7 @@ struct ResidentShared {
   // first sum warp may be writing the next round's.  That one's next write of
   // the same word lies behind a kBarStep that the sync warp takes part in
   int stop[2];
-  int status, iter, best, stalled;
+  int status, iter, best;
   int emax;                     // the last vector's largest biased exponent
   int ew[kRgMaxWarps];          // its worker warps'
   int fail;                     // a wait ran out
@@ -547,10 +547,12 @@ __device__ __forceinline__ void resident_body(const ResidentArgs& P, unsigned ch
   stamp(-1);
   const int all = nt + 32 * kRgServe;
   // the scale of m's digits (of its entries times their columns' powers of two):
-  // one place above the last vector's maximum (over an iteration m's grows by at most 1.3 and shrinks to no less than 0.3 on
-  // these systems); for the first m, which is like M^-1 A u, u's
-  auto next_scale = [](int emax) { return emax < kFxExpMin || emax > kFxExpMax ? kFxNone : emax - 1022 + 1; };
-  int E = next_scale(sh.emax);
+  // one place above the last vector's maximum, which shrinks by up to two places
+  // an iteration and hardly grows; for the first m, which is like M^-1 A u, u's.
+  // The second m is three places up: under loads on part of the body it grows by
+  // 1 to 4 places over the first (a product in FP64 instead: 19 us on 98k tets)
+  auto next_scale = [](int emax, int up) { return emax < kFxExpMin || emax > kFxExpMax ? kFxNone : emax - 1022 + up; };
+  int E = next_scale(sh.emax, 1), up = kFxSlack;
   if (worker) {
     double p = 0.0, q = 0.0, s = 0.0, z = 0.0, u_old = 0.0, alpha = 0.0, beta = 0.0;
     const int m_own = kRgRowBytes * (kRgRows * w + lane / 3) + 8 * rsub;   // cluster form: this lane's entry
@@ -589,7 +591,8 @@ __device__ __forceinline__ void resident_body(const ResidentArgs& P, unsigned ch
       const int top = sh.emax - 1022;          // 2^top is above m's scaled entries
       if (valid && (top > E || top < E - kFxSlack || !row_fx))
         n = row_product_m<CL>(P.A + 9 * (size_t)kb, cols, ke - kb, t10, rsub, P.m[par], (2 + par) * mrow);
-      E = next_scale(sh.emax);
+      E = next_scale(sh.emax, up);
+      up = 1;
       alpha = sh.ab[0];
       beta = sh.ab[1];
       z = fma(beta, z, n);
@@ -620,9 +623,11 @@ __device__ __forceinline__ void resident_body(const ResidentArgs& P, unsigned ch
     // sum warp j takes dot product j; the first forms the step lengths
     const int j = w - W - 1;
     double gam_inv = 0.0, den_k = 0.0;   // 1 / gamma and den / gamma^2 of the last iteration
-    // the third keeps count of the iterations without a smaller r.r (the first is
-    // what a round waits for): the iteration of the smallest, and its upper half
+    // the iteration of the smallest r.r and that one's upper half, for the next
+    // round's stop test.  Counted here, while the workers update (by the third sum
+    // warp, which no round waits for, an iteration took 0.35 us more on 98k tets)
     int best = 0, best_hi = 0x7fffffff;
+    bool stalled = false;
 #pragma unroll 1
     for (int it = 0;; it++) {
       bar_sync(kBarDots, nt + 96);
@@ -633,16 +638,7 @@ __device__ __forceinline__ void resident_body(const ResidentArgs& P, unsigned ch
       __syncwarp();
       if (j > 0) {
         bar_arrive(kBarTot, 96);
-        if (__double2hiint(t) < best_hi) {
-          best_hi = __double2hiint(t);
-          best = it;
-        }
         bar_sync(kBarStep, all);
-        if (j == 2 && lane == 0) {   // read behind the next kBarTot
-          sh.best = best;
-          sh.stalled = P.patience > 0 && it + 1 - best > P.patience + (best >> 2);
-        }
-        __syncwarp();
         if (sh.stop[it & 1]) break;
         continue;
       }
@@ -660,7 +656,7 @@ __device__ __forceinline__ void resident_body(const ResidentArgs& P, unsigned ch
         status = OD_ERR_NAN;
       } else if (!(rr > eps) || it >= P.max_iter) {
         stop = 1;
-      } else if (sh.stalled) {
+      } else if (stalled) {
         stop = 1;
         status = OD_ERR_NOT_CONVERGED;
       } else if (!isfinite(alpha) || !isfinite(beta)) {
@@ -676,11 +672,17 @@ __device__ __forceinline__ void resident_body(const ResidentArgs& P, unsigned ch
         if (stop) {
           sh.status = status;
           sh.iter = it;
+          sh.best = __double2hiint(rr) < best_hi ? it : best;
         }
       }
       __syncwarp();
       bar_sync(kBarStep, all);
       if (sh.stop[it & 1]) break;   // lane 0's word: the lanes' reads of fail may differ
+      if (__double2hiint(rr) < best_hi) {
+        best_hi = __double2hiint(rr);
+        best = it;
+      }
+      stalled = P.patience > 0 && it + 1 - best > P.patience + (best >> 2);
       gam_inv = 1.0 / t;
       den_k = den * gam_inv * gam_inv;
     }
@@ -723,7 +725,7 @@ __global__ void __launch_bounds__(32 * (MAXW + kRgServe), 1) pcg_resident_kernel
   __shared__ ResidentShared sh;
   if (threadIdx.x == 0) {
     sh.fail = 0;
-    sh.stop[0] = sh.stop[1] = sh.stalled = 0;
+    sh.stop[0] = sh.stop[1] = 0;
     sh.status = OD_OK;
     for (int k = 0; k < kPcgProfSlots; k++) sh.prof[k] = 0;
     if constexpr (CL)
