@@ -7,8 +7,8 @@
 // two signed digits X = h 2^29 + l, and a product takes three wide
 // multiply-adds (h h, h l, l h; l l is below the last place).  60 bits against
 // a row's sum of magnitudes and a vector's maximum, where FP64 keeps 53 against
-// every product: on the matrices and iterates of these solves the result is
-// within 0.7-1.6e-16 of the exact product in the 2-norm, FP64 within
+// every product: on the matrices and iterates of one-material solves the result
+// is within 0.7-1.6e-16 of the exact product in the 2-norm, FP64 within
 // 1.2-2.3e-16, as long as E is at most three binary places above the vector's
 // maximum (the caller checks that, and multiplies in FP64 otherwise).
 #pragma once

@@ -49,7 +49,7 @@ struct SolveScalars {           // device-resident PCG scalars
   double rz[2];                 // r.z by iteration parity
   double rr, bb, eps, rr0, tr_num, tr_den, alpha, beta;
   int iter, max_iter, done, status;
-  int best;                     // chip-resident form: the iteration of the smallest r.r
+  int best;                     // chip-resident form: the iteration at which r.r last had halved
 };
 
 struct SliceSys;
@@ -627,7 +627,8 @@ cudaError_t plan_malloc(T** p, size_t bytes) { return plan_malloc_bytes((void**)
 od_status resident_plan(Scene* s);
 void resident_free(ResidentPlan* R);
 od_status resident_ready(Scene* s);   // its device memory; called before resident_solve
-// patience: iterations without a smaller residual after which it gives up (OD_ERR_NOT_CONVERGED), 0: none
+// patience: iterations without r.r halving (and a quarter of those before) after which it gives up
+// (OD_ERR_NOT_CONVERGED), 0: none
 od_status resident_solve(Scene* s, const double* d_b, double* d_x, int pkind, double tol, int max_iter, int patience,
                          bool x_zero, unsigned long long* prof);
 // the one-launch fixed-point PCG of systems beyond the resident one (od_wide.cu)

@@ -29,10 +29,11 @@
 //
 // Microseconds per iteration, od_sparse.cu's persistent kernel (its pipelined
 // form: barrier, sums and product one after the other) -> the split above with
-// FP64 products -> this kernel: 108 DOFs 13.2 -> 3.3 -> 2.9, 2,160 DOFs 12.5 ->
-// 5.0 -> 3.5, 6,900 DOFs 12.9 -> 5.0 -> 5.6, 55,488 DOFs 16.7 -> 10.1 -> 8.3.
-// What is left is the dependent instructions of single warps (issue slots 20%
-// used, FP64 units 22% on the largest) and the grid barrier.
+// FP64 products -> this kernel: 108 DOFs 13.2 -> 3.3 -> 3.0, 2,160 DOFs 12.5 ->
+// 5.0 -> 3.5, 6,900 DOFs 12.9 -> 5.0 -> 5.7, 55,488 DOFs 16.7 -> 10.1 -> 8.4
+// (solves of 45 to 150 iterations, their start and end, 37 to 70 us, included).
+// What is left is the dependent instructions of single warps (issue slots 21%
+// used, FP64 units 24% on the largest) and the grid barrier.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -623,8 +624,8 @@ __device__ __forceinline__ void resident_body(const ResidentArgs& P, unsigned ch
     // sum warp j takes dot product j; the first forms the step lengths
     const int j = w - W - 1;
     double gam_inv = 0.0, den_k = 0.0;   // 1 / gamma and den / gamma^2 of the last iteration
-    // the iteration of the smallest r.r and that one's upper half, for the next
-    // round's stop test.  Counted here, while the workers update (by the third sum
+    // the iteration at which r.r last had halved, and its upper half then, for the
+    // next round's stop test.  Counted here, while the workers update (by the third sum
     // warp, which no round waits for, an iteration took 0.35 us more on 98k tets)
     int best = 0, best_hi = 0x7fffffff;
     bool stalled = false;
@@ -672,13 +673,13 @@ __device__ __forceinline__ void resident_body(const ResidentArgs& P, unsigned ch
         if (stop) {
           sh.status = status;
           sh.iter = it;
-          sh.best = __double2hiint(rr) < best_hi ? it : best;
+          sh.best = __double2hiint(rr) < best_hi - (1 << 20) ? it : best;
         }
       }
       __syncwarp();
       bar_sync(kBarStep, all);
       if (sh.stop[it & 1]) break;   // lane 0's word: the lanes' reads of fail may differ
-      if (__double2hiint(rr) < best_hi) {
+      if (__double2hiint(rr) < best_hi - (1 << 20)) {
         best_hi = __double2hiint(rr);
         best = it;
       }

@@ -3483,14 +3483,15 @@ od_status pcg_solve(Scene* s, const double* d_b, double* d_x, const od_solver_pa
       // ill-conditioned systems their residual parts from the true one or comes
       // down no further.  So (unless the form is asked for by name) the true
       // residual decides.  Above the tolerance, a pass goes on from it for up to
-      // 2% more iterations; a solve that this does not end, or that has not come
-      // down for 400 iterations and a quarter of those before, starts again in the
+      // 2% more iterations; a solve that this does not end, or whose r.r has not
+      // halved for 150 iterations and a quarter of those before, starts again in the
       // recurrence form, from the vector it was given.  Stiffness graded over 1e4,
-      // block-Jacobi, 1e-10 (emulated): 218 iterations there, none here; strewn
-      // stiffness comes down in steps of up to 192 iterations.
+      // block-Jacobi, 1e-10 (emulated): 218 iterations there, none here; solves on
+      // their way down stay above their best for up to 120 iterations with a
+      // preconditioner, and 190 of 1,500 without one.
       const bool decides = P.recur < 0;
       if (decides && !x_zero) OD_CUDA(cudaMemcpyAsync(P.r, d_x, sizeof(double) * (size_t)n, cudaMemcpyDeviceToDevice, strm));
-      OD_TRY(resident_solve(s, d_b, d_x, pk, prm->tol, prm->max_iter, decides ? 400 : 0, x_zero, profp));
+      OD_TRY(resident_solve(s, d_b, d_x, pk, prm->tol, prm->max_iter, decides ? 150 : 0, x_zero, profp));
       if (prof) OD_CUDA(cudaEventRecord(s->ctx->ev_pool[1], strm));
       if (!decides) return pcg_finish(s, d_b, d_x, shift, st, true, prof, phases);
       od_solve_stats ss{};
@@ -3499,7 +3500,8 @@ od_status pcg_solve(Scene* s, const double* d_b, double* d_x, const od_solver_pa
       // out of iterations on its way down: no fault of the form
       const SolveScalars& h = *P.sc_host;
       bool done = e != OD_OK || met() ||
-                  (ss.status == OD_ERR_NOT_CONVERGED && h.iter >= h.max_iter && h.iter - h.best <= 128 && h.tr_num <= 4.0 * h.rr);
+                  (ss.status == OD_ERR_NOT_CONVERGED && h.iter >= h.max_iter && h.iter - h.best <= std::max(64, h.iter / 8) &&
+                   h.tr_num <= 4.0 * h.rr);
       const int most = std::min(prm->max_iter, ss.iterations + std::max(2, ss.iterations / 50));
       while (!done && ss.status == OD_OK && ss.iterations < most) {
         const int used = ss.iterations;

@@ -15,10 +15,11 @@
 //   the shadow of the other warps' loads.
 //
 // An iteration, FP64 products before and this: 237,600 DOFs (94 MB of digits)
-// 42.5 -> 32.1 us, 424,320 (155 MB) 69.4 -> 45.9, 617,760 (300 MB) 87.0 ->
-// 69.9; of the 45.9 the product takes 27, at 5.6 TB/s (a plain read of as many
+// 42.5 -> 30.7 us, 424,320 (155 MB) 69.4 -> 46.4, 617,760 (300 MB) 87.0 ->
+// 69.9; of the 46.4 the product takes 27, at 5.6 TB/s (a plain read of as many
 // bytes: 21), its wait for the slowest CTA and the sum 8, the update 7.  The
-// digits cost a solve 81 us.  With the matrix loaded by the computing warps
+// digits and the products with x, in FP64, cost a solve 0.2 ms at the first size
+// and 0.3 at the second.  With the matrix loaded by the computing warps
 // instead of through a ring in shared memory a product took 54 us.
 #include <algorithm>
 #include <cmath>
