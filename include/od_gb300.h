@@ -160,7 +160,8 @@ typedef struct od_counters {
   double sweep_factor_ms;     /* their host time: rebuild of A in the reference layout, the
                                  factorisation and the upload of the sweep arrays */
   long long sweep_nnz;        /* strictly lower entries of the last factor */
-  long long sweep_applies;    /* applies timed while profiling is on */
+  long long sweep_applies;    /* applies timed while profiling is on (IC(0) in colour order: none, they
+                                 are inside the solve's one launch) */
   double sweep_apply_ms;      /* their summed CUDA-event durations */
   double sweep_apply_bytes;   /* their algorithmic bytes: 2 x (nnz x 12 B) + 7 x 8 B per row */
   long long sweep_levels;     /* dependency levels of the last factor's two sweeps (the apply's
